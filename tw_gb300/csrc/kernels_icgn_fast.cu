@@ -492,6 +492,116 @@ __device__ __forceinline__ bool pass_out_of_roi_warp(const Geom& g, const float*
     return __any_sync(0xffffffffu, out);
 }
 
+// Shared scratch of a POI held by one warp: rows of H^-1 (FP64), then the
+// right-hand side, the step dP and the new warp as they are exchanged between
+// the six lanes that compute them and all others.
+struct alignas(16) WarpScratch {
+    double h[36];
+    double b[6];
+    float dp[8];
+    float w[8];
+};
+
+__device__ __forceinline__ void load6(const float* s, float (&x)[6]) {
+    const float4 a = *reinterpret_cast<const float4*>(s);
+    const float2 b = *reinterpret_cast<const float2*>(s + 4);
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y;
+}
+
+// Ends one pass of a POI held by one warp: statistics, FP64 H^-1 b and the
+// warp update (coefficient k on lane k < 6; the other lanes repeat lane 5),
+// the convergence test on every lane, and the outputs when the POI is
+// finished.  v8: sum k of the pass on lanes 4k .. 4k+3; c: mean(R); st: the
+// POI's statistics.  The parameters P are those of the warp Wm: (W2, W0 - 1,
+// W1, W5, W3, W4 - 1).  Returns whether another pass follows, with its warp in
+// Wm.  Issue-bound like the sample loops: the exchanges go through shared
+// memory in words of 8 to 16 bytes, and no section runs on lane 0 alone.
+__device__ __forceinline__ bool warp_end_pass(const IcgnJob& jb, int p, int it, bool oor, float v8, float c,
+                                              float inv_s, const float* st, uint8_t rf, WarpScratch& sc,
+                                              float (&Wm)[6]) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const Geom& g = jb.g;
+    const int lane = threadIdx.x & 31, k6 = lane < 6 ? lane : 5;
+    const float S0 = __shfl_sync(FULL, v8, 0), S1 = __shfl_sync(FULL, v8, 4);
+    const float Ak = __shfl_sync(FULL, v8, 8 + 4 * k6);
+    const float m0 = S0 * inv_s;
+    const float mean_t = c + m0;
+    const float var = fmaf(-S0, m0, S1);
+    const float ts = sqrtf(var > 0.f ? var : 0.f);
+    int flag = kSuccess;
+    if (oor) {
+        flag = kOutofROI;
+    } else if (fabsf(mean_t) <= FLT_EPSILON || fabsf(ts) <= FLT_EPSILON) {
+        flag = kDarkSubset;
+    } else if (it == 0 && rf == kSingularHessian) {
+        flag = kSingularHessian;
+    }
+    bool cont = false;
+    if (flag == kSuccess) {
+        const float q = st[1] / ts;  // ||R - mean(R)|| / ||T - mean(T)||
+        const float bk = fmaf(q, fmaf(-m0, st[2 + k6], Ak), -st[8 + k6]);
+        if (lane < 6) sc.b[lane] = (double)bk;
+        __syncwarp();
+        const double2* hr = reinterpret_cast<const double2*>(sc.h + 6 * k6);
+        const double2* br = reinterpret_cast<const double2*>(sc.b);
+        double acc = 0.0;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const double2 h = hr[j], b = br[j];
+            acc = fma(h.x, b.x, acc);
+            acc = fma(h.y, b.y, acc);
+        }
+        if (lane < 6) sc.dp[lane] = (float)acc;
+        __syncwarp();
+        float dp[6];
+        load6(sc.dp, dp);
+        // W(P) o W(dP)^-1 (update_warp's operations), coefficient k on lane k:
+        // w_k = base_k + (x_k y_k - z_k v_k) / det
+        const float det = __fsub_rn(__fmul_rn(1.f + dp[1], 1.f + dp[5]), __fmul_rn(dp[2], dp[4]));
+        if (fabsf(det) <= FLT_EPSILON) {
+            flag = kSingularWarp;
+        } else {
+            const float a = __fsub_rn(__fsub_rn(__fmul_rn(dp[0], dp[4]), dp[3]), __fmul_rn(dp[3], dp[1]));
+            const float b = __fsub_rn(__fadd_rn(__fmul_rn(dp[0], dp[5]), dp[0]), __fmul_rn(dp[2], dp[3]));
+            const bool row1 = k6 >= 3;
+            const int r3 = row1 ? k6 - 3 : k6;  // 0: (1+d5, d4), 1: (1+d1, d2), 2: (a, b)
+            const float y = r3 == 0 ? 1.f + dp[5] : (r3 == 1 ? 1.f + dp[1] : a);
+            const float v = r3 == 0 ? dp[4] : (r3 == 1 ? dp[2] : b);
+            // row 0: (1 + P1, P2) for its first coefficient, (P2, 1 + P1) for
+            // the others; row 1: (P4, 1 + P5), then (1 + P5, P4)
+            const float e = 1.f + ((row1 ? Wm[4] : Wm[0]) - 1.f), f = row1 ? Wm[3] : Wm[1];
+            const bool ef = row1 != (r3 == 0);
+            const float x = ef ? e : f, z = ef ? f : e;
+            const float qw = __fdiv_rn(__fsub_rn(__fmul_rn(x, y), __fmul_rn(z, v)), det);
+            const float wk = r3 == 2 ? __fadd_rn(row1 ? Wm[5] : Wm[2], qw) : qw;
+            if (lane < 6) sc.w[lane] = wk;
+            __syncwarp();
+            load6(sc.w, Wm);
+            // scaled ||dP|| >= delta_p, squared, FP32
+            const float a1 = dp[1] * (float)g.rx, a2 = dp[2] * (float)g.ry;
+            const float a4 = dp[4] * (float)g.rx, a5 = dp[5] * (float)g.ry;
+            const float nrm2 = dp[0] * dp[0] + a1 * a1 + a2 * a2 + dp[3] * dp[3] + a4 * a4 + a5 * a5;
+            cont = it + 1 < g.max_iter && nrm2 >= g.delta_p * g.delta_p;
+        }
+    }
+    if (!cont && lane == 0) {
+        // finish: the counter is it+1 after a solve or an abort in a later
+        // pass; an abort in the first pass leaves it untouched
+        float* o = jb.p6 + (size_t)p * 6;
+        o[0] = Wm[2];
+        o[1] = Wm[0] - 1.f;
+        o[2] = Wm[1];
+        o[3] = Wm[5];
+        o[4] = Wm[3];
+        o[5] = Wm[4] - 1.f;
+        jb.flags[p] = (uint8_t)flag;
+        jb.u[p] = Wm[2];
+        jb.v[p] = Wm[5];
+        if (flag == kSuccess || it > 0) jb.iters[p] = it + 1;
+    }
+    return cont;
+}
+
 // Persistent IC-GN kernel, one POI per CTA at a time.  The target sampler:
 //   kSampWindow: the target window around the guess is staged in shared
 //     memory and interpolated with the separable Catmull-Rom weights;
@@ -800,17 +910,15 @@ __global__ void k_ref_grad(Geom g, const uint8_t* __restrict__ ref, float2* __re
 // POI is that of k_icgn_fast<32, ...>: the same sample order per lane, the
 // same sums, reduction, solve and update, so the results are identical.
 template <int NW, int SAMPLER, bool MULTI, int UNROLL>
-__global__ void __launch_bounds__(NW * 32, (NW >= 32 ? 1 : 32 / NW))
+__global__ void __launch_bounds__(NW * 32, NW == 4 ? 4 : 32 / NW)
     k_icgn_warp(const __grid_constant__ IcgnJobs J, int chunk) {
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ int s_next;
-    __shared__ double s_h[NW][36];  // rows of H^-1 of each warp's POI
-    __shared__ float s_p[NW][6];     // each warp's warp parameters P (lane 0)
+    __shared__ WarpScratch s_sc[NW];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (threadIdx.x == 0) s_next = 0;
     __syncthreads();
-    double* hw = s_h[wid];
-    float* pw = s_p[wid];
+    WarpScratch& sc = s_sc[wid];
     for (;;) {
         int t = 0;
         if (lane == 0) t = atomicAdd(&s_next, 1);
@@ -843,18 +951,14 @@ __global__ void __launch_bounds__(NW * 32, (NW >= 32 ? 1 : 32 / NW))
             }
             continue;
         }
-        // P in shared memory (lane 0 updates it); lane k < 6: row k of H^-1
-        // (FP64); the statistics are re-read at each solve, not held in
-        // registers through the sample loop
-        if (lane == 0) {
-            pw[0] = u0; pw[1] = 0.f; pw[2] = 0.f; pw[3] = v0; pw[4] = 0.f; pw[5] = 0.f;
-        }
+        // lane k < 6: row k of H^-1 (FP64); the statistics are re-read at each
+        // solve, not held in registers through the sample loop
         const float* st = jb.stats + (size_t)p * 16;
         const float c = st[0];
         if (lane < 6) {
             const double* hi = jb.hinv + (size_t)p * 21;
 #pragma unroll
-            for (int j = 0; j < 6; ++j) hw[lane * 6 + j] = hi[lane >= j ? tri(lane, j) : tri(j, lane)];
+            for (int j = 0; j < 6; ++j) sc.h[lane * 6 + j] = hi[lane >= j ? tri(lane, j) : tri(j, lane)];
         }
         __syncwarp();
         // sample k = lane + 32 j: its offset (dx, dy) and its column and row
@@ -874,9 +978,21 @@ __global__ void __launch_bounds__(NW * 32, (NW >= 32 ? 1 : 32 / NW))
                 const float4* smp = smp0;
                 const float2 w03 = make_float2(Wm[0], Wm[3]), w14 = make_float2(Wm[1], Wm[4]);
                 const float2 bxy = make_float2(bx, by);
-                if (it == 0) {
-                    // first pass: integer pixels (TW_paDIC_ICGN2D_CPU.cpp:609-637)
+                if (it == 0 && bx == truncf(bx) && by == truncf(by)) {
+                    // first pass (integer pixels, TW_paDIC_ICGN2D_CPU.cpp:609-637)
+                    // from a whole-pixel guess: the subset of the image shifted
+                    // by it, no coordinates
+                    const uint8_t* t0 = jb.tar + ((size_t)((int)by - g.ry) * g.pitch + ((int)bx - g.rx));
 #pragma unroll UNROLL
+                    for (int k = lane; k < S; k += 32) {
+                        const float4 e4 = __ldg(smp);
+                        smp += 32;
+                        const int ox = __float_as_int(e4.z), oy = __float_as_int(e4.w);
+                        ps.add((float)t0[oy * g.pitch + ox] - c, grad0[oy * g.rw + ox], make_float2(e4.x, e4.y));
+                    }
+                } else if (it == 0) {
+                    // first pass from a fractional guess: truncated coordinates
+#pragma unroll 2
                     for (int k = lane; k < S; k += 32) {
                         const float4 e4 = __ldg(smp);
                         smp += 32;
@@ -928,106 +1044,123 @@ __global__ void __launch_bounds__(NW * 32, (NW >= 32 ? 1 : 32 / NW))
                 ps.unpack(s);
                 v8 = warp_reduce8(s);
             }
-            // FP32 scalars, FP64 H^-1 b on lanes 0-5, warp update on lanes 0-5;
-            // sum k is held by lanes 4k .. 4k+3
-            const float S0 = __shfl_sync(FULL, v8, 0), S1 = __shfl_sync(FULL, v8, 4);
-            const float Ak = __shfl_sync(FULL, v8, 8 + 4 * (lane < 6 ? lane : 0));
-            const float m0 = S0 * inv_s;
-            const float mean_t = c + m0;
-            const float var = S1 - S0 * m0;
-            const float ts = sqrtf(var > 0.f ? var : 0.f);
-            int flag = kSuccess, cont = 0;
-            if (oor) {
-                flag = kOutofROI;
-            } else if (fabsf(mean_t) <= FLT_EPSILON || fabsf(ts) <= FLT_EPSILON) {
-                flag = kDarkSubset;
-            } else if (it == 0 && rf == kSingularHessian) {
-                flag = kSingularHessian;
-            }
-            float dpk = 0.f;
-            if (flag == kSuccess) {
-                const float q = st[1] / ts;  // ||R - mean(R)|| / ||T - mean(T)||
-                const float sumsd = lane < 6 ? st[2 + lane] : 0.f, qk = lane < 6 ? st[8 + lane] : 0.f;
-                const float bk = (lane < 6) ? q * (Ak - m0 * sumsd) - qk : 0.f;
-                const double bd = (double)bk;
-                double acc = 0.0;
-#pragma unroll
-                for (int j = 0; j < 6; ++j) {
-                    const double bj = __shfl_sync(FULL, bd, j);
-                    if (lane < 6) acc = fma(hw[lane * 6 + j], bj, acc);
-                }
-                dpk = (float)acc;
-            }
-            float dp[6];
-#pragma unroll
-            for (int j = 0; j < 6; ++j) dp[j] = __shfl_sync(FULL, dpk, j);
-            // W(P) o W(dP)^-1 (update_warp's operations), coefficient k on lane k:
-            // w_k = base_k + (x_k y_k - z_k v_k) / det
-            bool singular = false;
-            float wk = 0.f;
-            if (flag == kSuccess) {
-                const float P0 = pw[0], P1 = pw[1], P2 = pw[2], P3 = pw[3], P4 = pw[4], P5 = pw[5];
-                const float det = __fsub_rn(__fmul_rn(1.f + dp[1], 1.f + dp[5]), __fmul_rn(dp[2], dp[4]));
-                singular = fabsf(det) <= FLT_EPSILON;
-                if (!singular && lane < 6) {
-                    const float a = __fsub_rn(__fsub_rn(__fmul_rn(dp[0], dp[4]), dp[3]), __fmul_rn(dp[3], dp[1]));
-                    const float b = __fsub_rn(__fadd_rn(__fmul_rn(dp[0], dp[5]), dp[0]), __fmul_rn(dp[2], dp[3]));
-                    const int r3 = lane % 3;  // 0: (1+d5, d4), 1: (1+d1, d2), 2: (a, b)
-                    const float y = r3 == 0 ? 1.f + dp[5] : (r3 == 1 ? 1.f + dp[1] : a);
-                    const float v = r3 == 0 ? dp[4] : (r3 == 1 ? dp[2] : b);
-                    const float x = lane == 0 ? 1.f + P1 : (lane <= 2 ? P2 : (lane == 3 ? P4 : 1.f + P5));
-                    const float z = lane == 0 ? P2 : (lane <= 2 ? 1.f + P1 : (lane == 3 ? 1.f + P5 : P4));
-                    const float q = __fdiv_rn(__fsub_rn(__fmul_rn(x, y), __fmul_rn(z, v)), det);
-                    wk = lane == 2 ? __fadd_rn(P0, q) : (lane == 5 ? __fadd_rn(P3, q) : q);
-                }
-            }
-            float Wn[6];
-#pragma unroll
-            for (int j = 0; j < 6; ++j) Wn[j] = __shfl_sync(FULL, wk, j);
-            if (lane == 0) {
-                float P[6];
-#pragma unroll
-                for (int k = 0; k < 6; ++k) P[k] = pw[k];
-                if (flag == kSuccess) {
-                    if (singular) {
-                        flag = kSingularWarp;
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 6; ++k) Wm[k] = Wn[k];
-                        P[0] = Wn[2];
-                        P[1] = Wn[0] - 1.f;
-                        P[2] = Wn[1];
-                        P[3] = Wn[5];
-                        P[4] = Wn[3];
-                        P[5] = Wn[4] - 1.f;
-                        // scaled ||dP|| >= delta_p, squared, FP32
-                        const float a1 = dp[1] * (float)g.rx, a2 = dp[2] * (float)g.ry;
-                        const float a4 = dp[4] * (float)g.rx, a5 = dp[5] * (float)g.ry;
-                        const float nrm2 = dp[0] * dp[0] + a1 * a1 + a2 * a2 + dp[3] * dp[3] + a4 * a4 + a5 * a5;
-                        cont = (it + 1 < g.max_iter && nrm2 >= g.delta_p * g.delta_p) ? 1 : 0;
-                    }
-                }
-                if (!(flag == kSuccess && cont)) {
-                    // finish: the counter is it+1 after a solve or an abort in a
-                    // later pass; an abort in the first pass leaves it untouched
-                    jb.flags[p] = (uint8_t)flag;
-                    for (int k = 0; k < 6; ++k) jb.p6[(size_t)p * 6 + k] = P[k];
-                    jb.u[p] = P[0];
-                    jb.v[p] = P[3];
-                    if (flag == kSuccess || it > 0) jb.iters[p] = it + 1;
-                }
-#pragma unroll
-                for (int k = 0; k < 6; ++k) pw[k] = P[k];
-            }
-            cont = __shfl_sync(FULL, (flag == kSuccess && cont) ? 1 : 0, 0);
-            if (!cont) break;
-            // every lane has the new warp; lane 0's P is read by all at the next update
-#pragma unroll
-            for (int k = 0; k < 6; ++k) Wm[k] = Wn[k];
-            __syncwarp();
+            if (!warp_end_pass(jb, p, it, oor, v8, c, inv_s, st, rf, sc, Wm)) break;
             ++it;
         }
-        __syncwarp();  // hw is rewritten by the warp's next POI
+        __syncwarp();  // sc is rewritten by the warp's next POI
+    }
+}
+
+// IC-GN with one POI per CTA of NW warps, for launches of a few POIs per SM,
+// where one warp's sample steps follow each other with nothing to hide their
+// latency.  All threads interpolate
+// the pass's t' = T - mean(R) and its products with the gradient into shared
+// memory; the eight sums are then taken by one warp each, lane and order as in
+// k_icgn_warp (sample k on lane k % 32, then the same exchanges), so the
+// results are identical; warp 0 ends the pass.  It issues 2.3 times the
+// instructions of k_icgn_warp, so it is the faster one only on idle SMs.
+template <int NW, int SAMPLER, bool MULTI>
+__global__ void __launch_bounds__(NW * 32, 32 / NW) k_icgn_team(const __grid_constant__ IcgnJobs J) {
+    extern __shared__ __align__(16) float s_prod[];  // t', R_x t', R_y t' of the samples
+    __shared__ WarpScratch sc;
+    __shared__ float s_tot[8];
+    __shared__ int s_more[2];  // whether pass it (slot it % 2) is followed by another
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int pg = blockIdx.x;
+    int jj = 0;
+    if (MULTI) {
+        while (jj + 1 < J.njobs && pg >= J.job[jj + 1].begin) ++jj;
+    }
+    const IcgnJob& jb = J.job[jj];
+    const Geom& g = jb.g;
+    const int p = pg - jb.begin;
+    const int S = (2 * g.rx + 1) * (2 * g.ry + 1);
+    const float inv_s = 1.0f / (float)S;
+    const uint4* nb0 = static_cast<const uint4*>(jb.table) - ((size_t)g.sy * g.rw + g.sx);
+    const int2 pyx = jb.poi[p];
+    const int py = pyx.x, px = pyx.y;
+    const float u0 = jb.u[p], v0 = jb.v[p];
+    const uint8_t rf = jb.rflag[p];
+    if (rf == kDarkSubset || rf == kOutofROI) {
+        if (tid == 0) {
+            jb.flags[p] = rf;
+            const float P0[6] = {u0, 0.f, 0.f, v0, 0.f, 0.f};
+            for (int k = 0; k < 6; ++k) jb.p6[(size_t)p * 6 + k] = P0[k];
+        }
+        return;
+    }
+    const float* st = jb.stats + (size_t)p * 16;
+    const float c = st[0];
+    if (wid == 0 && lane < 6) {
+        const double* hi = jb.hinv + (size_t)p * 21;
+#pragma unroll
+        for (int j = 0; j < 6; ++j) sc.h[lane * 6 + j] = hi[lane >= j ? tri(lane, j) : tri(j, lane)];
+    }
+    __syncwarp();
+    const float2* grad0 = jb.grad + ((size_t)(py - g.ry - g.sy) * g.rw + (px - g.rx - g.sx));
+    float* s_t = s_prod;
+    float* s_a = s_prod + S;
+    float* s_b = s_prod + 2 * S;
+    float Wm[6] = {1.f, 0.f, u0, 0.f, 1.f, v0};
+    for (int it = 0;; ++it) {
+        const float bx = (float)px + Wm[2], by = (float)py + Wm[5];
+        const bool oor = pass_out_of_roi_warp(g, Wm, bx, by);
+        if (!oor) {
+            const float2 w03 = make_float2(Wm[0], Wm[3]), w14 = make_float2(Wm[1], Wm[4]), bxy = make_float2(bx, by);
+#pragma unroll 4
+            for (int k = tid; k < S; k += NW * 32) {
+                const float4 e4 = __ldg(jb.samples + k);
+                const int gofs = __float_as_int(e4.w) * g.rw + __float_as_int(e4.z);
+                const float2 wxy = __ffma2_rn(w03, make_float2(e4.x, e4.x),
+                                              __ffma2_rn(w14, make_float2(e4.y, e4.y), bxy));
+                const int ix = (int)wxy.x, iy = (int)wxy.y;
+                const float2 gr = grad0[gofs];
+                float tp;
+                if (it == 0) {
+                    // integer pixels (TW_paDIC_ICGN2D_CPU.cpp:609-637)
+                    tp = (float)jb.tar[(size_t)iy * g.pitch + ix] - c;
+                } else {
+                    const float2 f = __fadd2_rn(wxy, make_float2(-(float)ix, -(float)iy));
+                    const uint4 q = nb0[(unsigned)(iy * g.rw + ix)];
+                    if (SAMPLER == kSampNbhdBs) {
+                        tp = bs_combine4x4(bs_row_pair(q.x, q.y, f.x), bs_row_pair(q.z, q.w, f.x), f.y) - c;
+                    } else {
+                        tp = fmaf(0.5f, cr_combine4x4(cr_row_pair(q.x, q.y, f.x), cr_row_pair(q.z, q.w, f.x), f.y), -c);
+                    }
+                }
+                s_t[k] = tp;
+                s_a[k] = gr.x * tp;
+                s_b[k] = gr.y * tp;
+            }
+            __syncthreads();
+            // sum k of the pass in PassSums' order: t', t'^2, a, a dx, a dy, b, b dx, b dy
+            for (int k8 = wid; k8 < 8; k8 += NW) {
+                const float* x = k8 < 2 ? s_t : (k8 < 5 ? s_a : s_b);
+                float s = 0.f;
+                if (k8 == 1) {
+#pragma unroll 8
+                    for (int k = lane; k < S; k += 32) s = fmaf(x[k], x[k], s);
+                } else if (k8 == 0 || k8 == 2 || k8 == 5) {
+#pragma unroll 8
+                    for (int k = lane; k < S; k += 32) s += x[k];
+                } else {
+                    const float* d = reinterpret_cast<const float*>(jb.samples) + ((k8 == 3 || k8 == 6) ? 0 : 1);
+#pragma unroll 8
+                    for (int k = lane; k < S; k += 32) s = fmaf(x[k], __ldg(d + 4 * k), s);
+                }
+                s = warp_sum(s);
+                if (lane == 0) s_tot[k8] = s;
+            }
+            __syncthreads();
+        }
+        if (wid == 0) {
+            const float v8 = oor ? 0.f : s_tot[(lane >> 2) & 7];
+            const bool more = warp_end_pass(jb, p, it, oor, v8, c, inv_s, st, rf, sc, Wm);
+            if (lane == 0) s_more[it & 1] = more ? 1 : 0;
+        }
+        __syncthreads();
+        if (!s_more[it & 1]) break;
+        load6(sc.w, Wm);
     }
 }
 
@@ -1125,14 +1258,18 @@ cudaError_t launch_ref_grad(const Geom& g, const uint8_t* ref, float2* grad, cud
     return cudaGetLastError();
 }
 
+// unroll: the sample loops' unrolling, 2, 4 or, as "8", the deepest, which is
+// by 10 (2048^2, 41x41 subsets: 2.27 ms against 2.31 ms by 8 or 6 and 2.25 ms
+// by 13, which loses 10 % on 61x61 subsets); CTAs of fewer warps: by 4.
 template <int NW, int SAMPLER, bool MULTI>
 static cudaError_t launch_icgn_warp_t(const IcgnJobs& J, int chunk, int ctas_per_sm, int unroll, cudaStream_t st) {
-    // sample-loop unrolling: 2, 4 or 8 for the one-CTA-per-SM shape, 4 otherwise
     auto kern = k_icgn_warp<NW, SAMPLER, MULTI, 4>;
     if (NW == 32 && unroll == 2) kern = k_icgn_warp<NW, SAMPLER, MULTI, (NW == 32 ? 2 : 4)>;
-    if (NW == 32 && unroll == 8) kern = k_icgn_warp<NW, SAMPLER, MULTI, (NW == 32 ? 8 : 4)>;
-    // a few KB of shared memory: leave the rest of the SM's 256 KB to L1
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
+    if (NW == 32 && unroll == 8) kern = k_icgn_warp<NW, SAMPLER, MULTI, (NW == 32 ? 10 : 4)>;
+    // shared memory for the resident CTAs (up to 8 KB each with the runtime's
+    // 1 KB; at a share of 0 the smaller CTAs are not all resident), the rest of
+    // the SM's 256 KB to L1
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, NW == 32 ? 0 : 10);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0, occ = 0;
     cudaGetDevice(&dev);
@@ -1141,10 +1278,25 @@ static cudaError_t launch_icgn_warp_t(const IcgnJobs& J, int chunk, int ctas_per
     if (e != cudaSuccess) return e;
     if (ctas_per_sm > 0 && ctas_per_sm < occ) occ = ctas_per_sm;
     if (occ < 1) occ = 1;
+    // runs of at most `chunk` POIs, as many for every CTA: with runs of 32
+    // whatever the total, 1,936 POIs kept 61 of the 152 SMs busy
     long long grid = (long long)sms * occ;
-    const long long runs = ((long long)J.total + chunk - 1) / chunk;
-    if (grid > runs) grid = runs;
-    kern<<<(int)grid, NW * 32, 0, st>>>(J, chunk);
+    const long long rounds = std::max(1ll, ((long long)J.total + grid * chunk - 1) / (grid * chunk));
+    const int run = (int)(((long long)J.total + grid * rounds - 1) / (grid * rounds));
+    grid = std::min(grid, ((long long)J.total + run - 1) / run);
+    kern<<<(int)grid, NW * 32, 0, st>>>(J, run);
+    return cudaGetLastError();
+}
+
+template <int NW, int SAMPLER, bool MULTI>
+static cudaError_t launch_icgn_team_t(const IcgnJobs& J, cudaStream_t st) {
+    int S = 0;
+    for (int j = 0; j < J.njobs; ++j) S = std::max(S, (2 * J.job[j].g.rx + 1) * (2 * J.job[j].g.ry + 1));
+    const int smem = 3 * S * (int)sizeof(float);
+    auto kern = k_icgn_team<NW, SAMPLER, MULTI>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    kern<<<J.total, NW * 32, smem, st>>>(J);
     return cudaGetLastError();
 }
 
@@ -1176,7 +1328,24 @@ cudaError_t launch_icgn_fast_jobs(const IcgnJobs& J, int* work, const IcgnTune& 
     if (tune.sampler == kSampLut) { TWDIC_ICGN_WARP(NW, kSampLut); }                              \
     if (tune.sampler == kSampNbhdBs) { TWDIC_ICGN_WARP(NW, kSampNbhdBs); }                        \
     TWDIC_ICGN_WARP(NW, kSampNbhd)
-        if (tune.threads == 128) { TWDIC_ICGN_WARP_N(4); }
+        // The 32-warp CTAs (one per SM, 64 registers) are for launches that
+        // fill them.  Fewer POIs leave a warp's own latency in the open: up to 16
+        // per SM, CTAs of four warps at 128 registers, whose sample steps overlap
+        // more (1,936 POIs, 33x33 subsets: 44 us against 50 us), and up to four
+        // per SM the team kernel (285 POIs, 21x21 subsets: 23 us against 33 us;
+        // 1,936 POIs: 75 us).
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const bool full = tune.threads == 1024 && tune.sampler != kSampLut;
+        if (full && J.total <= 4 * sms) {
+#define TWDIC_ICGN_TEAM(SA)                                                                                \
+    return multi ? launch_icgn_team_t<8, SA, true>(J, st) : launch_icgn_team_t<8, SA, false>(J, st)
+            if (tune.sampler == kSampNbhdBs) { TWDIC_ICGN_TEAM(kSampNbhdBs); }
+            TWDIC_ICGN_TEAM(kSampNbhd);
+#undef TWDIC_ICGN_TEAM
+        }
+        if (tune.threads == 128 || (full && J.total <= 16 * sms)) { TWDIC_ICGN_WARP_N(4); }
         if (tune.threads == 256) { TWDIC_ICGN_WARP_N(8); }
         if (tune.threads == 512) { TWDIC_ICGN_WARP_N(16); }
         TWDIC_ICGN_WARP_N(32);
