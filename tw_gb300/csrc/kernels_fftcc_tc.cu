@@ -1697,10 +1697,18 @@ cudaError_t launch_fftcc_tc_jobs(const FftccJob* jobs, int njobs, const FftccTun
 #undef TWDIC_TC_CASE
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem_bytes);
     if (e != cudaSuccess) return e;
+    // fewer batches than the SMs' groups: groups spread over half of the SMs
+    // (36 batches of 20x20 windows: 27 us in 36 CTAs of one group, 33 us in 8 of
+    // five).  Over all of them a launch of 277 batches is 4 us faster still, but
+    // keeps other streams' kernels off every SM.
+    const int spread = (2 * nb + sms - 1) / sms;
+    if (spread < s.groups) {
+        s.smem_bytes -= (s.groups - spread) * s.group_bytes;
+        s.groups = spread;
+    }
     e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) return e;
-    // one CTA per SM holds two groups when shared memory allows; with one
-    // group, two CTAs share an SM when they fit
+    // with one group per CTA, two CTAs share an SM when they fit
     const int threads = kThreads * s.groups;
     int occ = 1;
     if (s.groups == 1 && 2 * (s.smem_bytes + 2048) <= 228 * 1024) occ = 2;
