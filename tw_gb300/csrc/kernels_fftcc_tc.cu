@@ -85,6 +85,9 @@ struct TcShape {
     int tiles4;  // 128-row tiles of the surface (stage 4)
     int FS;      // complex values per cached spectrum row: N rounded up to 4
     int NW4;  // 32-bit words per window row in the exact re-evaluation
+    // x / N and x / H for x < 512 as (x rcp) >> 16, rcp = 65536 / d rounded up
+    // (exact: x (rcp d - 65536) < 512 * 64 < 65536)
+    unsigned rcpN, rcpH;
     int lo;   // 1: twiddles as FP16 hi + lo (two MMAs per product), 0: hi only
     // shared twiddle tables
     int off_b1h, off_b1l, off_c2h, off_c2l, off_s2h, off_s2l, off_b4h, off_b4l, tab_bytes;
@@ -161,6 +164,12 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
+
+// The words of such a descriptor apart: sdesc_lo(a) + (d >> 4) is that of the
+// address a + d (addresses are below 2^18: no carry leaves the field).
+__device__ __forceinline__ uint32_t sdesc_lo(uint32_t saddr, uint32_t lbo) { return (saddr >> 4) | (lbo >> 4) << 16; }
+__device__ __forceinline__ uint32_t sdesc_hi(uint32_t sbo) { return sbo >> 4 | 1u << 14; }
+__device__ __forceinline__ uint64_t sdesc_of(uint32_t lo, uint32_t hi) { return (uint64_t)hi << 32 | lo; }
 
 __host__ __device__ constexpr uint32_t idesc_f16(int n, bool neg_b) {
     // kind::f16: D f32 (bit 4), A = B = f16, both K-major, N>>3 at bit 17, M>>4 at bit 24
@@ -388,6 +397,8 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
     const uint32_t gaddr = smem_u32(gbase);
     const uint32_t sbase = smem_u32(sm);
     const int FS = s.FS;  // cached spectrum: complex values per (POI, ky) row
+    auto divN = [&](int x) { return (int)(((unsigned)x * s.rcpN) >> 16); };
+    auto divH = [&](int x) { return (int)(((unsigned)x * s.rcpH) >> 16); };
     // the job (image pair, POI set) of a batch: batches of job j are
     // [batch_begin_j, batch_begin_j + ceil(n_j / PB))
     auto job_of = [&](int bt) {
@@ -494,6 +505,9 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
         if (t < 2 * kMaxPB * 2) (&cs.wsum[grp][0][0])[t] = 0;
         if (t < PB) cs.smaxv[grp][t] = 0u;
         // this batch's windows (staged one batch earlier)
+        // (each wait below: the threads agree that none gave up at the next
+        // barrier they need anyway; until then a late MMA could only spoil
+        // operands and accumulators that nothing uses any more)
         bool ok = mbar_wait(&cs.mbar_tma[grp][sl], (tphase >> sl) & 1u);
         tphase ^= 1u << sl;
         if (group_sync_or(bar_id, !ok)) { abort_group(false, sl ^ 1); return false; }
@@ -508,7 +522,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
         // warp reductions.  Rows past the batch's windows are not written
         // (the rows of D1 they give are never read).
         for (int rr = t; rr < s.tiles1 * 128; rr += 128) {
-            const int pw = rr / N, y = rr - pw * N;
+            const int pw = divN(rr), y = rr - pw * N;
             const int wi = 2 * pw + (REF ? 0 : 1);
             const bool inb = pw < PB;
             const bool data = inb && cs.spoi[grp][sl][pw].x >= 0;
@@ -564,14 +578,15 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
         // ---- stage 1: D1[(w,y)][(part,kx)] = A1 * B1 (the real DFT along x)
         if (t == 0) {
             tc_fence_after();
+            const uint32_t hi = sdesc_hi(16 * K1);
+            const uint32_t a0 = sdesc_lo(gaddr + s.off_a13, 128);
+            const uint32_t bh0 = sdesc_lo(sbase + s.off_b1h, 128), bl0 = sdesc_lo(sbase + s.off_b1l, 128);
             for (int tile = 0; tile < s.tiles1; ++tile) {
-                const uint32_t a0 = gaddr + s.off_a13 + tile * (128 * K1 * 2);
+#pragma unroll
                 for (int kk = 0; kk < K1 / 16; ++kk) {
-                    const uint64_t a = sdesc(a0 + kk * 256, 128, 16 * K1);
-                    const uint64_t bh = sdesc(sbase + s.off_b1h + kk * 256, 128, 16 * K1);
-                    const uint64_t bl = sdesc(sbase + s.off_b1l + kk * 256, 128, 16 * K1);
-                    mma_f16(tm + tile * 2 * HP, a, bh, idesc_f16(2 * HP, false), kk > 0);
-                    if (LO) mma_f16(tm + tile * 2 * HP, a, bl, idesc_f16(2 * HP, false), 1);
+                    const uint64_t a = sdesc_of(a0 + tile * (128 * K1 * 2 / 16) + kk * 16, hi);
+                    mma_f16(tm + tile * 2 * HP, a, sdesc_of(bh0 + kk * 16, hi), idesc_f16(2 * HP, false), kk > 0);
+                    if (LO) mma_f16(tm + tile * 2 * HP, a, sdesc_of(bl0 + kk * 16, hi), idesc_f16(2 * HP, false), 1);
                 }
             }
             mma_commit(mbar);
@@ -591,7 +606,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
         }
         ok = mbar_wait(mbar, phase);
         phase ^= 1u;
-        if (group_sync_or(bar_id, !ok)) { abort_group(pending, sl ^ 1); return false; }
+        __syncwarp();  // the TMEM reads below are warp-wide
         tc_fence_after();
 
         // ---- epilogue 1: D1 -> A2 (rows (p, kx); K = (y, part) interleaved
@@ -615,7 +630,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
             if (s.z2part) group_sync(bar_id);
             for (int tile = 0; tile < s.tiles1; ++tile) {
                 const int rr = tile * 128 + t;
-                const int p = rr / N, y = rr - p * N;
+                const int p = divN(rr), y = rr - p * N;
                 const bool data = p < PB;
                 uint8_t* rowp = a2 + (data ? p * H : 0) * 16 +
                                 (LO ? (y >> 3) * LB2 + (y & 7) * 2 : (y >> 2) * LB2 + (y & 3) * 4);
@@ -651,7 +666,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
         }
         tc_fence_before();
         fence_async_smem();
-        group_sync(bar_id);
+        if (group_sync_or(bar_id, !ok)) { abort_group(pending, sl ^ 1); return false; }
 
         // ---- stage 2: F = Y * W (rows (p,kx); columns Re ky | Im ky), K
         // steps over the data columns only
@@ -661,12 +676,15 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
             const uint32_t a2 = gaddr + s.off_a2;
             if (!LO) {
                 // K = (y, part) interleaved: one MMA per output part and K step
-                for (int kk = 0; kk < s.ks2; ++kk) {
-                    const uint64_t a = sdesc(a2 + 2 * kk * LB2, LB2, 128);
-                    const uint64_t wr = sdesc(sbase + s.off_w2re + kk * 256, 128, 32 * NP);
-                    const uint64_t wi = sdesc(sbase + s.off_w2im + kk * 256, 128, 32 * NP);
-                    mma_f16(tm, a, wr, idesc_f16(NP, false), kk > 0);       // Re = Yr cos + Yi sin
-                    mma_f16(tm + NP, a, wi, idesc_f16(NP, false), kk > 0);  // Im = -Yr sin + Yi cos
+                const uint32_t ahi = sdesc_hi(128), whi = sdesc_hi(32 * NP);
+                const uint32_t a0 = sdesc_lo(a2, LB2), da = LB2 / 8;
+                const uint32_t wr = sdesc_lo(sbase + s.off_w2re, 128), wi = sdesc_lo(sbase + s.off_w2im, 128);
+#pragma unroll
+                for (int kk = 0; kk < NP / 8; ++kk) {
+                    if (kk >= s.ks2) break;
+                    const uint64_t a = sdesc_of(a0 + kk * da, ahi);
+                    mma_f16(tm, a, sdesc_of(wr + kk * 16, whi), idesc_f16(NP, false), kk > 0);       // Re = Yr cos + Yi sin
+                    mma_f16(tm + NP, a, sdesc_of(wi + kk * 16, whi), idesc_f16(NP, false), kk > 0);  // Im = -Yr sin + Yi cos
                 }
             }
             for (int kk = 0; LO && kk < s.ks2; ++kk) {
@@ -692,7 +710,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
         // reference row is read from L2 while stage 2 runs (with split
         // twiddles chunk by chunk in epilogue 2: registers)
         const bool rowv2 = t < PB * H;
-        const int p2 = rowv2 ? t / H : 0, ky2 = rowv2 ? t - p2 * H : 0;
+        const int p2 = rowv2 ? divH(t) : 0, ky2 = rowv2 ? t - p2 * H : 0;
         const bool live2 = rowv2 && !REF && !cs.sdark[grp][p2];
         const uint4* frow = reinterpret_cast<const uint4*>(jb.fspec + ((size_t)(live2 ? b0 + p2 : 0) * H + ky2) * FS);
         uint4 fr[LO ? 1 : NP / 4];
@@ -703,7 +721,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
         }
         ok = mbar_wait(mbar, phase);
         phase ^= 1u;
-        if (group_sync_or(bar_id, !ok)) { abort_group(pending, sl ^ 1); return false; }
+        __syncwarp();  // the TMEM reads below are warp-wide
         tc_fence_after();
 
         if (REF) {
@@ -730,7 +748,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
             if (t < PB && b0 + t < n_job) jb.fsum[b0 + t] = make_int2(cs.wsum[grp][2 * t][0], cs.wsum[grp][2 * t][1]);
             tc_fence_before();
             if (t == 0) cs.snext[grp] = nxt;
-            group_sync(bar_id);
+            if (group_sync_or(bar_id, !ok)) { abort_group(pending, sl ^ 1); return false; }
             cur = nb;
             nb = cs.snext[grp];
             sl ^= 1;
@@ -804,19 +822,22 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
         }
         tc_fence_before();
         fence_async_smem();
-        group_sync(bar_id);
+        if (group_sync_or(bar_id, !ok)) { abort_group(pending, sl ^ 1); return false; }
 
         // ---- stage 3: conj(Z) = conj(C) * W (rows (p,kx); columns Re v | Im v)
         if (t == 0) {
             tc_fence_after();
             const int K3 = s.k3w;
             if (!LO) {
-                for (int kk = 0; kk < s.ks2; ++kk) {
-                    const uint64_t a = sdesc(gaddr + s.off_a13 + kk * 256, 128, 16 * K3);
-                    const uint64_t wr = sdesc(sbase + s.off_w2re + kk * 256, 128, 32 * NP);
-                    const uint64_t wi = sdesc(sbase + s.off_w2im + kk * 256, 128, 32 * NP);
-                    mma_f16(tm, a, wr, idesc_f16(NP, false), kk > 0);
-                    mma_f16(tm + NP, a, wi, idesc_f16(NP, false), kk > 0);
+                const uint32_t ahi = sdesc_hi(16 * K3), whi = sdesc_hi(32 * NP);
+                const uint32_t a0 = sdesc_lo(gaddr + s.off_a13, 128);
+                const uint32_t wr = sdesc_lo(sbase + s.off_w2re, 128), wi = sdesc_lo(sbase + s.off_w2im, 128);
+#pragma unroll
+                for (int kk = 0; kk < NP / 8; ++kk) {
+                    if (kk >= s.ks2) break;
+                    const uint64_t a = sdesc_of(a0 + kk * 16, ahi);
+                    mma_f16(tm, a, sdesc_of(wr + kk * 16, whi), idesc_f16(NP, false), kk > 0);
+                    mma_f16(tm + NP, a, sdesc_of(wi + kk * 16, whi), idesc_f16(NP, false), kk > 0);
                 }
             }
             for (int kk = 0; LO && kk < s.ks2; ++kk) {
@@ -840,7 +861,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
         }
         ok = mbar_wait(mbar, phase);
         phase ^= 1u;
-        if (group_sync_or(bar_id, !ok)) { abort_group(pending, sl ^ 1); return false; }
+        __syncwarp();  // the TMEM reads below are warp-wide
         tc_fence_after();
 
         // ---- epilogue 3: D3 -> A4 (rows (p, v), K = (kx, part) interleaved:
@@ -859,7 +880,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
                 if (s.z4part) group_sync(bar_id);
             }
             const bool rowv = t < PB * H;
-            const int p = rowv ? t / H : 0, ky = rowv ? t - (t / H) * H : 0;
+            const int p = rowv ? divH(t) : 0, ky = rowv ? t - p * H : 0;
             const float wgt = (ky == 0 || 2 * ky == N) ? 1.f : 2.f;
             uint8_t* rowp = a4 + (p * N) * 16 + (ky >> 2) * LB4 + (ky & 3) * 4;
             // TMEM reads three 8-column chunks at a time, one wait each
@@ -890,26 +911,28 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
         }
         tc_fence_before();
         fence_async_smem();
-        group_sync(bar_id);
+        if (group_sync_or(bar_id, !ok)) { abort_group(pending, sl ^ 1); return false; }
 
         // ---- stage 4: c[(p,v)][u] = A4 * B4 (the c2r inverse along kx)
         if (t == 0) {
             tc_fence_after();
             const int LB4 = s.lbo4;
+            const uint32_t ahi = sdesc_hi(128), bhi = sdesc_hi(16 * K4);
+            const uint32_t a0 = sdesc_lo(gaddr + s.off_a4, LB4), da = LB4 / 8;
+            const uint32_t bh0 = sdesc_lo(sbase + s.off_b4h, 128), bl0 = sdesc_lo(sbase + s.off_b4l, 128);
             for (int tile = 0; tile < s.tiles4; ++tile) {
-                for (int kk = 0; kk < K4 / 16; ++kk) {
-                    const uint64_t a = sdesc(gaddr + s.off_a4 + tile * 2048 + 2 * kk * LB4, LB4, 128);
-                    const uint64_t bh = sdesc(sbase + s.off_b4h + kk * 256, 128, 16 * K4);
-                    const uint64_t bl = sdesc(sbase + s.off_b4l + kk * 256, 128, 16 * K4);
-                    mma_f16(tm + tile * NP, a, bh, idesc_f16(NP, false), kk > 0);
-                    if (LO) mma_f16(tm + tile * NP, a, bl, idesc_f16(NP, false), 1);
+#pragma unroll
+                for (int kk = 0; kk < HP / 8; ++kk) {  // K4 = 2 HP
+                    const uint64_t a = sdesc_of(a0 + tile * (2048 / 16) + kk * da, ahi);
+                    mma_f16(tm + tile * NP, a, sdesc_of(bh0 + kk * 16, bhi), idesc_f16(NP, false), kk > 0);
+                    if (LO) mma_f16(tm + tile * NP, a, sdesc_of(bl0 + kk * 16, bhi), idesc_f16(NP, false), 1);
                 }
             }
             mma_commit(mbar);
         }
         ok = mbar_wait(mbar, phase);
         phase ^= 1u;
-        if (group_sync_or(bar_id, !ok)) { abort_group(pending, sl ^ 1); return false; }
+        __syncwarp();  // the TMEM reads below are warp-wide
         tc_fence_after();
 
         // ---- epilogue 4: approximate peak, candidates, exact re-evaluation
@@ -929,7 +952,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
             if (k >= ntile) break;
             const int R = 128 * k + t;
             const bool rowv = R < PB * N;
-            const int p4 = rowv ? R / N : 0;
+            const int p4 = rowv ? divN(R) : 0;
             const bool live = rowv && !cs.sdark[grp][p4];
             float bv = -3.4e38f;
 #pragma unroll
@@ -938,16 +961,17 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
                 float cv[8];
                 tmem_ld8(tm_warp + k * NP + y0, cv);
                 tmem_ld_wait();
+                // (columns past N in the last chunk are zero: the twiddle rows
+                // are; a peak is never below the surface's mean of zero)
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (live && y0 + j < N && cv[j] > bv) bv = cv[j];
+                for (int j = 0; j < 8; j += 2) bv = fmaxf(bv, fmaxf(cv[j], cv[j + 1]));
             }
             const unsigned seg = __match_any_sync(kFull, live ? p4 : -1);
             const uint32_t ov = __reduce_max_sync(seg, f32_ord(bv));
             if (live && lane == __ffs(seg) - 1) atomicMax(&cs.smaxv[grp][p4], ov);
             bvk[k] = bv;
         }
-        group_sync(bar_id);
+        if (group_sync_or(bar_id, !ok)) { abort_group(pending, sl ^ 1); return false; }
         // candidates: every shift within kCandZncc (ZNCC units; the surface is
         // N^2 ZNCC) of the approximate peak, the peak itself included, as one
         // bit per y of each row; a warp with no such row skips the second read
@@ -957,7 +981,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
             if (k >= ntile) break;
             const int R = 128 * k + t;
             const bool rowv = R < PB * N;
-            const int p4 = rowv ? R / N : 0;
+            const int p4 = rowv ? divN(R) : 0;
             const bool live = rowv && !cs.sdark[grp][p4];
             const float th = live ? f32_unord(cs.smaxv[grp][p4]) - kCandZncc * (float)n2 : 3.4e38f;
             if (__any_sync(kFull, live && bvk[k] >= th)) {
@@ -970,9 +994,11 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
-                        if (live && y0 + j < N && cv[j] >= th) m |= 1ull << (y0 + j);
+                        if (cv[j] >= th) m |= 1ull << (y0 + j);
                 }
-                cmk[k] = m;
+                // not the columns past N, nor rows without a POI (their
+                // accumulators are of operands nobody wrote: any value)
+                cmk[k] = live ? m & (~0ull >> (64 - N)) : 0ull;
             }
         }
         tc_fence_before();
@@ -1011,7 +1037,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
             if (k >= ntile) break;
             const int R = 128 * k + t;
             if (R < PB * N) {
-                const int p4 = R / N, x4 = R - p4 * N;
+                const int p4 = divN(R), x4 = R - p4 * N;
                 if (x4 == 0) cs.cbase[grp][p4] = exk[k];
                 if (x4 == N - 1) cs.cend[grp][p4] = exk[k] + cnk[k];
             }
@@ -1034,7 +1060,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
             for (int k = 0; k < 2; ++k) {
                 if (cnk[k] > 0 && exk[k] < lo + kCandChunk && exk[k] + cnk[k] > lo) {
                     const int R = 128 * k + t;
-                    const int p4 = R / N, x4 = R - p4 * N;
+                    const int p4 = divN(R), x4 = R - p4 * N;
                     uint64_t m = cmk[k];
                     for (int q = exk[k]; m != 0; ++q) {
                         const int y = __ffsll((long long)m) - 1;
@@ -1339,6 +1365,8 @@ bool make_shape(const Geom& g, const FftccTune& tune, TcShape& s) {
     // per-group regions: one operand region shared by A1, A2, A3, A4 and the
     // peak scratch, then the windows
     s.NW4 = (N + 3) / 4;
+    s.rcpN = (65536u + N - 1) / N;
+    s.rcpH = (65536u + s.H - 1) / s.H;
     // stages 2 and 3 take K over the data columns only: (y, part) interleaved
     // 2N with single twiddles, N per part block with split ones
     s.ks2 = s.lo ? (N + 15) / 16 : (2 * N + 15) / 16;
