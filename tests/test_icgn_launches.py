@@ -55,5 +55,7 @@ def test_launch_shapes_bit_identical(w, h, r, grid, margin, guessed, interp):
     a = _run(ref, pair.tar, p, interp, False, guess)
     b = _run(ref, pair.tar, p, interp, True, guess)
     for k in a:
+        if guessed and k == "zncc":
+            continue  # not an output of a guessed frame
         np.testing.assert_array_equal(a[k], b[k], err_msg=k)
     assert (a["flags"] == 0).any()

@@ -218,6 +218,16 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
@@ -763,6 +773,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
         {
             if (s.z4early) zero_a4_padding(gbase + s.off_a4, s, PB * N, t);
             const float sc = live2 ? cs.sscale[grp][p2] : 0.f;
+            const float2 sc2 = make_float2(sc, sc);
             const int K3 = s.k3w;
             uint8_t* a3 = gbase + s.off_a13;
 #pragma unroll
@@ -781,17 +792,25 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
                     fb = fr[LO ? 0 : (c >> 2) + 1];
                 }
                 const uint32_t fw[8] = {fa.x, fa.y, fa.z, fa.w, fb.x, fb.y, fb.z, fb.w};
+                // conj(C), which feeds the forward matrices of stage 3, two
+                // columns at a time on the packed FP32 pipe; past N both spectra
+                // are zero (zero rows of the twiddle matrix, zero cache columns)
                 float br[8], bi[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&fw[i]));
-                    const int kx = c + i;
-                    float cr = (f.x * gr[i] + f.y * gi[i]) * sc;
-                    float ci = (f.x * gi[i] - f.y * gr[i]) * sc;
-                    if (kx >= N || (ky2 == 0 && kx == 0)) { cr = 0.f; ci = 0.f; }
-                    br[i] = cr;
-                    bi[i] = -ci;  // conj(C) feeds the forward matrices of stage 3
+                for (int i = 0; i < 8; i += 2) {
+                    const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&fw[i]));
+                    const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&fw[i + 1]));
+                    const float2 fx = make_float2(f0.x, f1.x), fy = make_float2(f0.y, f1.y);
+                    const float2 g_r = make_float2(gr[i], gr[i + 1]), g_i = make_float2(gi[i], gi[i + 1]);
+                    const float2 nfx = __fmul2_rn(fx, make_float2(-1.f, -1.f));
+                    const float2 cr = __fmul2_rn(__ffma2_rn(fx, g_r, __fmul2_rn(fy, g_i)), sc2);
+                    const float2 ci = __fmul2_rn(__ffma2_rn(nfx, g_i, __fmul2_rn(fy, g_r)), sc2);
+                    br[i] = cr.x;
+                    br[i + 1] = cr.y;
+                    bi[i] = ci.x;
+                    bi[i + 1] = ci.y;
                 }
+                if (c == 0 && ky2 == 0) br[0] = bi[0] = 0.f;  // the means' product
                 if (rowv2) {
                     uint4 q;
                     if (LO) {  // K = (part, ky)
@@ -883,30 +902,19 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
             const int p = rowv ? divH(t) : 0, ky = rowv ? t - p * H : 0;
             const float wgt = (ky == 0 || 2 * ky == N) ? 1.f : 2.f;
             uint8_t* rowp = a4 + (p * N) * 16 + (ky >> 2) * LB4 + (ky & 3) * 4;
-            // TMEM reads three 8-column chunks at a time, one wait each
-            // (columns N .. NP-1 are padding)
-#pragma unroll
-            for (int cb = 0; cb < NP; cb += 24) {
-                if (cb >= N) break;
-                float re[24], im[24];
-#pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    if (cb + 8 * q < NP) {
-                        tmem_ld8(tm_warp + cb + 8 * q, re + 8 * q);
-                        tmem_ld8(tm_warp + NP + cb + 8 * q, im + 8 * q);
-                    }
-                }
+            // 16 columns a turn (columns N .. NP-1 are padding)
+            const float nwgt = -wgt;
+#pragma unroll 1
+            for (int cb = 0; cb < N; cb += 16) {
+                float re[16], im[16];
+                tmem_ld16(tm_warp + cb, re);
+                tmem_ld16(tm_warp + NP + cb, im);
                 tmem_ld_wait();
-                if (rowv) {
+                uint8_t* q = rowp + cb * 16;
+                const int left = rowv ? N - cb : 0;
 #pragma unroll
-                    for (int j = 0; j < 24; ++j) {
-                        const int x = cb + j;
-                        if (x < NP && x < N) {
-                            // Zi = -D_i
-                            *reinterpret_cast<uint32_t*>(rowp + x * 16) = pack2(wgt * re[j], -wgt * im[j]);
-                        }
-                    }
-                }
+                for (int j = 0; j < 16; ++j)
+                    if (j < left) *reinterpret_cast<uint32_t*>(q + j * 16) = pack2(wgt * re[j], nwgt * im[j]);  // Zi = -D_i
             }
         }
         tc_fence_before();
@@ -954,17 +962,17 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
             const bool rowv = R < PB * N;
             const int p4 = rowv ? divN(R) : 0;
             const bool live = rowv && !cs.sdark[grp][p4];
+            // (16 columns a turn, rolled: the kernel is larger than the
+            // instruction cache.  Columns past N are zero, as the twiddle rows
+            // are, and a peak is never below the surface's mean of zero)
             float bv = -3.4e38f;
-#pragma unroll
-            for (int y0 = 0; y0 < NP; y0 += 8) {
-                if (y0 >= N) break;  // padding columns
-                float cv[8];
-                tmem_ld8(tm_warp + k * NP + y0, cv);
+#pragma unroll 1
+            for (int y0 = 0; y0 < NP; y0 += 16) {
+                float cv[16];
+                tmem_ld16(tm_warp + k * NP + y0, cv);
                 tmem_ld_wait();
-                // (columns past N in the last chunk are zero: the twiddle rows
-                // are; a peak is never below the surface's mean of zero)
 #pragma unroll
-                for (int j = 0; j < 8; j += 2) bv = fmaxf(bv, fmaxf(cv[j], cv[j + 1]));
+                for (int j = 0; j < 16; j += 2) bv = fmaxf(bv, fmaxf(cv[j], cv[j + 1]));
             }
             const unsigned seg = __match_any_sync(kFull, live ? p4 : -1);
             const uint32_t ov = __reduce_max_sync(seg, f32_ord(bv));
@@ -986,15 +994,16 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
             const float th = live ? f32_unord(cs.smaxv[grp][p4]) - kCandZncc * (float)n2 : 3.4e38f;
             if (__any_sync(kFull, live && bvk[k] >= th)) {
                 uint64_t m = 0ull;
-#pragma unroll
-                for (int y0 = 0; y0 < NP; y0 += 8) {
-                    if (y0 >= N) break;  // padding columns
-                    float cv[8];
-                    tmem_ld8(tm_warp + k * NP + y0, cv);
+#pragma unroll 1
+                for (int y0 = 0; y0 < NP; y0 += 16) {
+                    float cv[16];
+                    tmem_ld16(tm_warp + k * NP + y0, cv);
                     tmem_ld_wait();
+                    uint32_t m16 = 0u;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        if (cv[j] >= th) m |= 1ull << (y0 + j);
+                    for (int j = 0; j < 16; ++j)
+                        if (cv[j] >= th) m16 |= 1u << j;
+                    m |= (uint64_t)m16 << y0;
                 }
                 // not the columns past N, nor rows without a POI (their
                 // accumulators are of operands nobody wrote: any value)
@@ -1075,15 +1084,17 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
             {
                 const int NW4 = s.NW4;
                 const uint32_t tail = (N & 3) ? (0xffffffffu >> (8 * (4 - (N & 3)))) : 0xffffffffu;
-                const int rot = lane % NW4;
                 const int rs = cs.wrs[grp][sl];
                 const bool wsm = cs.wsm[grp][sl] != 0;
                 // task (c, y) = y nc + c for thread t, stepped by 128: a
                 // warp's lanes take the candidates of one row side by side
                 // (windows of different POIs: their rows fall in different
                 // banks), one shared atomic per task
-                const int dy = 128 / nc, dc = 128 - dy * nc;
-                int y = t / nc, c = t - (t / nc) * nc;
+                // (quotients of at most 128 by a reciprocal: x + 1/2 is far from
+                // the multiples)
+                const float rnc = __frcp_rn((float)nc);
+                const int dy = (int)(128.5f * rnc), dc = 128 - dy * nc;
+                int y = (int)(((float)t + 0.5f) * rnc), c = t - y * nc;
                 for (; y < N;) {
                     unsigned acc0 = 0u, acc1 = 0u;
                     {
@@ -1091,7 +1102,6 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
                         const int p = code >> 16, ky = (code >> 8) & 0xff, kx = code & 0xff;
                         int yy = y + ky;
                         if (yy >= N) yy -= N;
-                        int j = rot;
                         if (wsm) {
                             // the staged boxes: the circular row product as
                             // two linear segments, f[0, N - kx) g[kx, N) and
@@ -1104,7 +1114,8 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
                             const uint8_t* fb = cs.wptr[grp][sl][2 * p] + y * rs;
                             const uint8_t* gb = cs.wptr[grp][sl][2 * p + 1] + yy * rs;
                             const uint32_t g0 = ld_unaligned_p(gb);
-#pragma unroll 2
+                            int j = lane % NW4;
+#pragma unroll 1
                             for (int jj = 0; jj < NW4; ++jj) {
                                 uint32_t fw = ld_unaligned_p(fb + 4 * j);
                                 if (j == NW4 - 1) fw &= tail;
@@ -1135,7 +1146,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
                 const int a = max(cs.cbase[grp][t], lo), b = min(cs.cend[grp][t], lo + kCandChunk);
                 for (int k = a; k < b; ++k) {
                     const int code = ps->cand[k - lo];
-                    const int sc = ps->candS[k - lo], id = ((code >> 8) & 0xff) * N + (code & 0xff);
+                    const int sc = ps->candS[k - lo], id = code & 0xffff;  // (v, u): the order of v N + u
                     if (sc > best_s || (sc == best_s && id < best_i)) {
                         best_s = sc;
                         best_i = id;
@@ -1152,7 +1163,7 @@ __device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape&
             if (cs.sdark[grp][t]) {
                 status[gp] = 1;  // dark subset: outputs untouched (TW_paDIC_FFTCC2D_CPU.cpp:272-275)
             } else {
-                int iu = best_i % N, iv = best_i / N;
+                int iu = best_i & 0xff, iv = best_i >> 8;
                 if (iu > g.rx) iu -= N;
                 if (iv > g.ry) iv -= N;
                 const long long sf = cs.wsum[grp][2 * t][0], sg = cs.wsum[grp][2 * t + 1][0];
