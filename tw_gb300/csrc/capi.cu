@@ -299,16 +299,50 @@ struct Engine {
         return TWDIC_OK;
     }
 
-    // FFT-CC of all POIs into device arrays.
-    int fftcc(float* u, float* v, float* z, uint8_t* st) {
+    bool fftcc_on_tc() const {
+        return prm.path == TWDIC_PATH_FAST && fftcc_tune.use_tc && fftcc_tc_supported(g);
+    }
+
+    // What a frame needs before its FFT-CC, in one launch: the outputs that
+    // start at zero (a frame starts from zero displacements for dark FFT-CC
+    // subsets and a zero iteration count, as a freshly calloc'd reference
+    // buffer would), the neighbourhood table of IC-GN, the work counters.  The
+    // per-reference pass of FFT-CC comes first: it uses the counters too.
+    int begin_frame(float* u, float* v, float* z, int* iters, bool with_icgn) {
+        if (fftcc_on_tc()) TW_TRY(ensure_fspec(fftcc_tune));
+        PrepJob pj{};
+        pj.g = g;
+        pj.tar = d_tar.as<uint8_t>();
+        pj.n = n;
+        pj.zero_f[0] = u;
+        pj.zero_f[1] = v;
+        pj.zero_f[2] = z;
+        pj.zero_i = iters;
+        const bool table = with_icgn && uses_neighbourhoods();
+        if (table) {
+            TW_TRY(d_lut.ensure(sizeof(uint4) * (size_t)g.rw * g.rh));
+            pj.table = d_lut.as<uint4>();
+            pj.full = solve_tune().sampler == kSampNbhdBs ? 1 : 0;
+        }
+        PrepJobsT<1> J;
+        J.counters = d_work.as<int>();
+        J.ncounters = 2;
+        add_prep_job(J, pj);
+        TW_CUDA(launch_prepare(J, stream));
+        if (with_icgn && !table) TW_TRY(prepare_target());
+        return TWDIC_OK;
+    }
+
+    // FFT-CC of all POIs into device arrays; begun: after begin_frame.
+    int fftcc(float* u, float* v, float* z, uint8_t* st, bool begun = false) {
         if (!have_ref || !have_tar) return fail(TWDIC_ERR_STATE, "FFT-CC needs a reference and a target image");
         const int2* poi = d_poi.as<int2>();
-        if (prm.path == TWDIC_PATH_FAST && fftcc_tune.use_tc && fftcc_tc_supported(g)) {
+        if (fftcc_on_tc()) {
             TW_TRY(ensure_fspec(fftcc_tune));
             TW_TRY(ensure_tc_maps(fftcc_tune));
             TW_CUDA(launch_fftcc_tc(g, d_ref.as<uint8_t>(), d_tar.as<uint8_t>(), d_tcmaps.p, tcmaps.key, tcmaps.uw,
                                     tcmaps.utoff, c_fspec.as<uint32_t>(), c_fsum.as<int2>(), poi, n, u, v, z, st,
-                                    d_err.as<unsigned>(), d_work.as<int>() + 1, fftcc_tune, stream));
+                                    d_err.as<unsigned>(), d_work.as<int>() + 1, fftcc_tune, stream, false, begun));
         } else {
             TW_CUDA(launch_fftcc_plain(g, d_ref.as<uint8_t>(), d_tar.as<uint8_t>(), poi, n, d_tw.as<float2>(), u, v, z,
                                        st, stream));
@@ -355,20 +389,30 @@ struct Engine {
     // LUT of the target or its 4x4 neighbourhood table.
     int prepare_target() {
         if (!have_ref || !have_tar) return fail(TWDIC_ERR_STATE, "IC-GN needs a reference and a target image");
-        if (interp == TWDIC_INTERP_BSPLINE && prm.path == TWDIC_PATH_FAST && solve_tune().sampler == kSampNbhdBs) {
+        if (uses_neighbourhoods()) {
             TW_TRY(d_lut.ensure(sizeof(uint4) * (size_t)g.rw * g.rh));
-            TW_CUDA(launch_nbhd_table(g, d_tar.as<uint8_t>(), d_lut.as<uint4>(), stream, true));
+            PrepJob pj{};
+            pj.g = g;
+            pj.tar = d_tar.as<uint8_t>();
+            pj.table = d_lut.as<uint4>();
+            pj.full = solve_tune().sampler == kSampNbhdBs ? 1 : 0;
+            PrepJobsT<1> J;
+            add_prep_job(J, pj);
+            TW_CUDA(launch_prepare(J, stream));
         } else if (interp == TWDIC_INTERP_BSPLINE) {
             TW_TRY(d_lut.ensure(sizeof(float4) * 4 * (size_t)g.rw * g.rh));
             TW_CUDA(launch_bspline_lut(g, d_tar.as<uint8_t>(), d_lut.as<float4>(), stream));
         } else if (prm.path == TWDIC_PATH_PLAIN || icgn_tune.sampler == kSampLut) {
             TW_TRY(d_lut.ensure(sizeof(float4) * 4 * (size_t)g.rw * g.rh));
             TW_CUDA(launch_bicubic_lut(g, d_tar.as<uint8_t>(), d_lut.as<float4>(), stream));
-        } else if (icgn_tune.sampler == kSampNbhd) {
-            TW_TRY(d_lut.ensure(sizeof(uint4) * (size_t)g.rw * g.rh));
-            TW_CUDA(launch_nbhd_table(g, d_tar.as<uint8_t>(), d_lut.as<uint4>(), stream));
         }
         return TWDIC_OK;
+    }
+
+    // whether IC-GN reads the neighbourhood table
+    bool uses_neighbourhoods() const {
+        const int s = solve_tune().sampler;
+        return prm.path == TWDIC_PATH_FAST && (s == kSampNbhd || s == kSampNbhdBs);
     }
 
     // the fast IC-GN launch shape; B-spline from the neighbourhood table
@@ -665,16 +709,10 @@ int twdic_frame_process(twdic_frame* h, const uint8_t* tar, int32_t stride, int 
     const bool cached = e.cache_valid;
     TW_TRY(e.ensure_cache(nullptr));
     TW_CUDA(cudaEventRecord(e.ev[2], e.stream));
-    // a frame starts from zero displacements for dark FFT-CC subsets and a
-    // zero iteration count, as a freshly calloc'd reference buffer would
-    TW_CUDA(cudaMemsetAsync(du, 0, 4 * n, e.stream));
-    TW_CUDA(cudaMemsetAsync(dv, 0, 4 * n, e.stream));
-    TW_CUDA(cudaMemsetAsync(dz, 0, 4 * n, e.stream));
-    TW_CUDA(cudaMemsetAsync(dit, 0, 4 * n, e.stream));
-    TW_TRY(e.fftcc(du, dv, dz, e.d_fst.as<uint8_t>()));
-    TW_CUDA(cudaEventRecord(e.ev[3], e.stream));
-    TW_TRY(e.prepare_target());
+    TW_TRY(e.begin_frame(du, dv, dz, dit, true));
     TW_CUDA(cudaEventRecord(e.ev[6], e.stream));
+    TW_TRY(e.fftcc(du, dv, dz, e.d_fst.as<uint8_t>(), true));
+    TW_CUDA(cudaEventRecord(e.ev[3], e.stream));
     TW_TRY(e.icgn_solve(du, dv, dp6, dit, dfl));
     TW_CUDA(cudaEventRecord(e.ev[4], e.stream));
     if (!dev) {
@@ -758,14 +796,14 @@ int twdic_frame_phase_times(const twdic_frame* hc, float* t6) {
         float a = 0, b = 0, c = 0, d = 0, f = 0, pr = 0;
         TW_CUDA(cudaEventElapsedTime(&a, e.ev[0], e.ev[1]));
         TW_CUDA(cudaEventElapsedTime(&f, e.ev[1], e.ev[2]));
-        TW_CUDA(cudaEventElapsedTime(&b, e.ev[2], e.ev[3]));
-        TW_CUDA(cudaEventElapsedTime(&pr, e.ev[3], e.ev[6]));
-        TW_CUDA(cudaEventElapsedTime(&c, e.ev[6], e.ev[4]));
+        TW_CUDA(cudaEventElapsedTime(&pr, e.ev[2], e.ev[6]));
+        TW_CUDA(cudaEventElapsedTime(&b, e.ev[6], e.ev[3]));
+        TW_CUDA(cudaEventElapsedTime(&c, e.ev[3], e.ev[4]));
         TW_CUDA(cudaEventElapsedTime(&d, e.ev[4], e.ev[5]));
         const bool cached = e.last_times[5] < 0.f;
         e.last_times[0] = a;
         e.last_times[1] = b;
-        e.last_times[2] = pr;  // target LUT
+        e.last_times[2] = pr;  // target table, zeroed outputs
         e.last_times[3] = c;
         e.last_times[4] = d;
         e.last_times[5] = cached ? 0.f : f;
@@ -1188,19 +1226,14 @@ int batch_sampler(const IcgnTune& tune, const Engine& e) {
     return tune.sampler == kSampNbhd ? kSampNbhdBs : kSampLut;
 }
 
-// The frame's per-frame target table for its sampler.
-int prepare_target_for(Engine& e, int sampler) {
+// The frame's float LUT for the LUT sampler.
+int prepare_lut(Engine& e) {
     const Geom& g = e.g;
-    if (sampler == kSampLut) {
-        TW_TRY(e.d_lut.ensure(sizeof(float4) * 4 * (size_t)g.rw * g.rh));
-        if (e.interp == TWDIC_INTERP_BSPLINE)
-            TW_CUDA(launch_bspline_lut(g, e.d_tar.as<uint8_t>(), e.d_lut.as<float4>(), e.stream));
-        else
-            TW_CUDA(launch_bicubic_lut(g, e.d_tar.as<uint8_t>(), e.d_lut.as<float4>(), e.stream));
-    } else if (sampler == kSampNbhd || sampler == kSampNbhdBs) {
-        TW_TRY(e.d_lut.ensure(sizeof(uint4) * (size_t)g.rw * g.rh));
-        TW_CUDA(launch_nbhd_table(g, e.d_tar.as<uint8_t>(), e.d_lut.as<uint4>(), e.stream, sampler == kSampNbhdBs));
-    }
+    TW_TRY(e.d_lut.ensure(sizeof(float4) * 4 * (size_t)g.rw * g.rh));
+    if (e.interp == TWDIC_INTERP_BSPLINE)
+        TW_CUDA(launch_bspline_lut(g, e.d_tar.as<uint8_t>(), e.d_lut.as<float4>(), e.stream));
+    else
+        TW_CUDA(launch_bicubic_lut(g, e.d_tar.as<uint8_t>(), e.d_lut.as<float4>(), e.stream));
     return TWDIC_OK;
 }
 
@@ -1260,17 +1293,14 @@ int batch_enqueue(twdic_batch* b, const BatchArgs& a) {
         if (fast) fast_ic.push_back(i);
         prep.push_back(pj);
     }
+    // the per-reference pass of a frame's FFT-CC runs on its own counters
+    for (int i : fast_tc) TW_TRY(a.frames[i]->e.ensure_fspec(b->fftcc_tune));
     for (size_t k0 = 0; k0 < prep.size(); k0 += kMaxPrepJobs) {
         PrepJobs P;
-        for (size_t k = k0; k < prep.size() && k < k0 + kMaxPrepJobs; ++k) {
-            PrepJob& pj = P.job[P.njobs++];
-            pj = prep[k];
-            pj.px_begin = P.px_total;
-            pj.z_begin = P.z_total;
-            if (pj.table) P.px_total += (long long)pj.g.rw * pj.g.rh;
-            P.z_total += pj.n;
-        }
-        TW_CUDA(launch_batch_prepare(P, b->stream));
+        P.counters = b->d_work.as<int>();
+        P.ncounters = 2 + kMaxTcSegsScratch;
+        for (size_t k = k0; k < prep.size() && k < k0 + kMaxPrepJobs; ++k) add_prep_job(P, prep[k]);
+        TW_CUDA(launch_prepare(P, b->stream));
     }
     TW_TRY(mark(1));
     // FFT-CC of the frames off the tensor-core path, one call each
@@ -1284,6 +1314,7 @@ int batch_enqueue(twdic_batch* b, const BatchArgs& a) {
     // the frames in segments of one window size), per kMaxTcJobsPerLaunch frames
     {
         std::vector<FftccJob> jobs;
+        bool zeroed = true;  // the counters, by the preparation launch
         for (size_t m = 0; m < fast_tc.size(); ++m) {
             const int i = fast_tc[m];
             Engine& e = a.frames[i]->e;
@@ -1295,7 +1326,8 @@ int batch_enqueue(twdic_batch* b, const BatchArgs& a) {
                                     o.v, o.z, e.d_fst.as<uint8_t>()});
             if ((int)jobs.size() == kMaxTcJobsPerLaunch || m + 1 == fast_tc.size()) {
                 TW_CUDA(launch_fftcc_tc_jobs(jobs.data(), (int)jobs.size(), b->fftcc_tune, b->d_err.as<unsigned>(),
-                                             b->d_work.as<int>() + 1, b->stream));
+                                             b->d_work.as<int>() + 1, b->stream, false, zeroed));
+                zeroed = false;
                 jobs.clear();
             }
         }
@@ -1305,8 +1337,7 @@ int batch_enqueue(twdic_batch* b, const BatchArgs& a) {
     for (int i = 0; i < count; ++i) {
         Engine& e = a.frames[i]->e;
         if (e.prm.path == TWDIC_PATH_FAST) {
-            const int sampler = batch_sampler(b->tune, e);
-            if (sampler == kSampLut) TW_TRY(prepare_target_for(e, sampler));
+            if (batch_sampler(b->tune, e) == kSampLut) TW_TRY(prepare_lut(e));
         } else {
             TW_TRY(e.prepare_target());
         }
@@ -1630,14 +1661,11 @@ int twdic_tracker_process(twdic_tracker* t, const uint8_t* img, int32_t stride, 
     TW_TRY(e.set_tar(img, stride, mem_in));
     float* du = t->d_last_u.as<float>();
     float* dv = t->d_last_v.as<float>();
-    TW_CUDA(cudaMemsetAsync(du, 0, 4 * n, e.stream));
-    TW_CUDA(cudaMemsetAsync(dv, 0, 4 * n, e.stream));
-    TW_CUDA(cudaMemsetAsync(e.d_zncc.p, 0, 4 * n, e.stream));
-    TW_CUDA(cudaMemsetAsync(e.d_iters.p, 0, 4 * n, e.stream));
     TW_TRY(e.ensure_cache(nullptr));
-    TW_TRY(e.fftcc(du, dv, e.d_zncc.as<float>(), e.d_fst.as<uint8_t>()));
+    TW_TRY(e.begin_frame(du, dv, e.d_zncc.as<float>(), e.d_iters.as<int>(), t->with_icgn != 0));
+    TW_TRY(e.fftcc(du, dv, e.d_zncc.as<float>(), e.d_fst.as<uint8_t>(), true));
     if (t->with_icgn) {
-        TW_TRY(e.icgn(du, dv, e.d_p6.as<float>(), e.d_iters.as<int>(), e.d_flags.as<uint8_t>()));
+        TW_TRY(e.icgn_solve(du, dv, e.d_p6.as<float>(), e.d_iters.as<int>(), e.d_flags.as<uint8_t>()));
     } else {
         TW_CUDA(cudaMemsetAsync(e.d_flags.p, 0, n, e.stream));
     }

@@ -53,11 +53,14 @@ struct IcgnJob {
     int n;      // POIs of the job
     int begin;  // first global POI index of the job
 };
-struct IcgnJobs {
+// (a launch of one job passes a table of one: 21 KB of parameters otherwise)
+template <int N>
+struct IcgnJobsT {
     int njobs = 0;
     int total = 0;  // POIs of all jobs
-    IcgnJob job[kMaxJobs];
+    IcgnJob job[N];
 };
+using IcgnJobs = IcgnJobsT<kMaxJobs>;
 static_assert(sizeof(IcgnJobs) < 32000, "IC-GN job table exceeds the kernel parameter limit");
 
 // Launch shape of the tensor-core FFT-CC kernel.
@@ -77,13 +80,11 @@ cudaError_t launch_ref_precompute_plain(const Geom& g, const uint8_t* ref, const
 cudaError_t launch_bicubic_lut(const Geom& g, const uint8_t* tar, float4* lut, cudaStream_t st);
 // B-spline coefficient LUT of the target, same layout (kernels_plain.cu)
 cudaError_t launch_bspline_lut(const Geom& g, const uint8_t* tar, float4* lut, cudaStream_t st);
-// 4x4 byte neighbourhoods of every ROI pixel of the target (kernels_icgn_fast.cu);
-// full: the last ROI row and column too, bytes outside the image zero (the
-// B-spline sampler), otherwise those entries are zero (the bicubic samplers)
-cudaError_t launch_nbhd_table(const Geom& g, const uint8_t* tar, uint4* table, cudaStream_t st, bool full = false);
-// One frame of a batch's preparation launch (kernels_icgn_fast.cu): its
-// neighbourhood table (table null: none) and the output arrays set to zero
-// (null: left alone), n entries each.
+// One frame of a preparation launch (kernels_icgn_fast.cu): its
+// neighbourhood table (null: none; full: every ROI pixel, bytes outside the
+// image zero, for the B-spline sampler, otherwise the last ROI row and column
+// zero, for the bicubic ones) and the output arrays set to zero (null: left
+// alone), n entries each.
 struct PrepJob {
     Geom g;
     const uint8_t* tar;
@@ -92,17 +93,33 @@ struct PrepJob {
     float* zero_f[3];    // u, v, zncc
     int* zero_i;         // iteration counters
     int n;
-    long long px_begin;  // first table item of the frame
+    long long px_begin;  // first table item of the frame (kPrepRows table rows of one column)
     long long z_begin;   // first zeroing item of the frame
 };
 constexpr int kMaxPrepJobs = 128;
-struct PrepJobs {
+constexpr int kPrepRows = 8;
+template <int N>
+struct PrepJobsT {
     int njobs = 0;
     long long px_total = 0, z_total = 0;
-    PrepJob job[kMaxPrepJobs];
+    int* counters = nullptr;  // work counters of the launches that follow, set to zero (null: none)
+    int ncounters = 0;
+    PrepJob job[N];
 };
+using PrepJobs = PrepJobsT<kMaxPrepJobs>;
 static_assert(sizeof(PrepJobs) < 32000, "preparation table exceeds the kernel parameter limit");
-cudaError_t launch_batch_prepare(const PrepJobs& jobs, cudaStream_t st);
+// Appends a frame: its items are numbered after those of the jobs before it.
+template <int N>
+void add_prep_job(PrepJobsT<N>& J, const PrepJob& in) {
+    PrepJob& j = J.job[J.njobs++];
+    j = in;
+    j.px_begin = J.px_total;
+    j.z_begin = J.z_total;
+    if (j.table) J.px_total += (long long)j.g.rw * ((j.g.rh + kPrepRows - 1) / kPrepRows);
+    J.z_total += j.n;
+}
+cudaError_t launch_prepare(const PrepJobs& jobs, cudaStream_t st);
+cudaError_t launch_prepare(const PrepJobsT<1>& job, cudaStream_t st);
 cudaError_t launch_icgn_plain(const Geom& g, const uint8_t* tar, const int2* poi, int n, const float* subR,
                               const float2* sd, const float* chol, const float* refnorm, const uint8_t* rflag,
                               const float4* lut, float* u, float* v, float* p6, int* iters, uint8_t* flags,
@@ -150,14 +167,15 @@ uint64_t fftcc_tc_maps_key(const Geom& g, const FftccTune& tune);
 bool fftcc_tc_encode_maps(const Geom& g, const uint8_t* ref, const uint8_t* tar, const FftccTune& tune,
                           void* host_buf, TcMapInfo* info);
 // err: error flags; work: scratch -- one int (one window size) or kMaxTcSegsScratch
-// ints (several), zeroed by the launcher
+// ints (several), zeroed by the launcher unless `zeroed` says that they are zero
 // The reference windows' spectra are cached per reference: fspec [n][N/2+1][FS]
 // FP16 (Re, Im) pairs with FS = N rounded up to 4 (fftcc_tc_spectrum_bytes),
 // fsum [n] the windows' (sum f, sum f^2).  ref = true runs the per-reference
 // pass that writes them; ref = false the per-frame FFT-CC that reads them.
 cudaError_t launch_fftcc_tc(const Geom& g, const uint8_t* ref_img, const uint8_t* tar_img, const void* maps,
                             uint64_t map_key, int uw, int utoff, uint32_t* fspec, int2* fsum, const int2* poi, int n, float* u, float* v, float* zncc, uint8_t* status,
-                            unsigned* err, int* work, const FftccTune& tune, cudaStream_t st, bool ref = false);
+                            unsigned* err, int* work, const FftccTune& tune, cudaStream_t st, bool ref = false,
+                            bool zeroed = false);
 size_t fftcc_tc_spectrum_bytes(const Geom& g, int n);
 // One image pair of a batched tensor-core FFT-CC launch.  Jobs of one window
 // size share one k_fftcc_tc launch; jobs of several window sizes (up to 32)
@@ -181,7 +199,7 @@ struct FftccJob {
     uint8_t* status;
 };
 cudaError_t launch_fftcc_tc_jobs(const FftccJob* jobs, int njobs, const FftccTune& tune, unsigned* err, int* work,
-                                 cudaStream_t st, bool ref = false);
+                                 cudaStream_t st, bool ref = false, bool zeroed = false);
 bool fftcc_tc_supported(const Geom& g);
 
 // ---- tracking loop (kernels_track.cu)

@@ -126,11 +126,13 @@ struct TcJob {
     int n;            // POIs of the job
     int batch_begin;  // first batch index of the job within its segment
 };
-struct TcJobs {
+template <int N>
+struct TcJobsT {  // (a launch of one job passes a table of one)
     int njobs;
     int nbatch;  // batches of all jobs (one window size) or of the first segment
-    TcJob job[kMaxTcJobs];
+    TcJob job[N];
 };
+using TcJobs = TcJobsT<kMaxTcJobs>;
 // A segment of a mixed-size launch: its shape, twiddle tables and jobs
 // [job_lo, job_hi); CTAs [cta_begin, next segment's cta_begin) start on it.
 struct TcSeg {
@@ -341,7 +343,8 @@ struct TcCta {
 // The tensor maps of jobs [lo, hi): visible to the tensor-map proxy (they
 // were written to device memory by copies) and prefetched.  Thread 0 of each
 // group issues the group's TMA copies, so each such thread fences.
-__device__ __forceinline__ void tc_acquire_maps(const TcJobs& J, int lo, int hi) {
+template <class Jobs>
+__device__ __forceinline__ void tc_acquire_maps(const Jobs& J, int lo, int hi) {
     for (int j = lo; j < hi; ++j) {
         const TcMaps* m = J.job[j].maps;
         const CUtensorMap* mm[2] = {&m->ref_u, &m->tar_u};
@@ -385,8 +388,8 @@ __device__ __forceinline__ void zero_a4_padding(uint8_t* a4, const TcShape& s, i
             *reinterpret_cast<uint4*>(a4 + c * s.lbo4 + r * 16) = make_uint4(0, 0, 0, 0);
 }
 
-template <int NP, int HP, bool MULTI, bool LO, bool REF>
-__device__ __forceinline__ bool tc_group_batches(const TcJobs& J, const TcShape& s, int job_lo, int job_hi,
+template <int NP, int HP, bool MULTI, bool LO, bool REF, class Jobs>
+__device__ __forceinline__ bool tc_group_batches(const Jobs& J, const TcShape& s, int job_lo, int job_hi,
                                                  int nbatch, int first, int* counter, int counter_base,
                                                  unsigned* err, TcCta& cs, uint8_t* sm, uint32_t& phase,
                                                  uint32_t& tphase) {
@@ -1231,7 +1234,7 @@ __device__ __forceinline__ void tc_teardown(TcCta& cs, uint32_t tmem_cols) {
 // of every group by position, then the next free one from the launch-wide
 // counter, which evens out the groups' finishing times.
 template <int NP, int HP, bool MULTI, bool LO, bool REF>
-__global__ void __launch_bounds__(NP <= 48 ? 128 * kMaxGroups : 128 * kSegGroups, 1) k_fftcc_tc(const __grid_constant__ TcJobs J, TcShape s,
+__global__ void __launch_bounds__(NP <= 48 ? 128 * kMaxGroups : 128 * kSegGroups, 1) k_fftcc_tc(const __grid_constant__ TcJobsT<MULTI ? kMaxTcJobs : 1> J, TcShape s,
                                                                  const uint4* __restrict__ tables, unsigned* err,
                                                                  int* work) {
     extern __shared__ __align__(1024) uint8_t sm[];
@@ -1611,7 +1614,7 @@ int shape_index(const TcShape& s) {
 // Jobs of several window sizes in one k_fftcc_tc_seg launch.  counters:
 // kMaxTcSegs ints of scratch.
 cudaError_t launch_segments(const FftccJob* jobs, int njobs, const FftccTune& tune, unsigned* err, int* counters,
-                            cudaStream_t st) {
+                            cudaStream_t st, bool zeroed) {
     // jobs grouped by window size (stable)
     std::vector<int> order(njobs);
     for (int j = 0; j < njobs; ++j) order[j] = j;
@@ -1669,38 +1672,27 @@ cudaError_t launch_segments(const FftccJob* jobs, int njobs, const FftccTune& tu
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(counters, 0, sizeof(int) * kMaxTcSegs, st);
-    if (e != cudaSuccess) return e;
+    if (!zeroed) {
+        e = cudaMemsetAsync(counters, 0, sizeof(int) * kMaxTcSegs, st);
+        if (e != cudaSuccess) return e;
+    }
     kern<<<sms, kThreads * kSegGroups, smem, st>>>(*J, *S, err, counters);
     return cudaGetLastError();
 }
 
-}  // namespace
-
-cudaError_t launch_fftcc_tc_jobs(const FftccJob* jobs, int njobs, const FftccTune& tune, unsigned* err, int* work,
-                                 cudaStream_t st, bool ref) {
-    // the per-reference pass runs with single twiddles whatever the tuning
-    // (its spectra are rounded to FP16 when cached)
-    FftccTune tn = tune;
-    if (ref) tn.twiddle_lo = 0;
-    if (njobs < 1 || njobs > kMaxTcJobs) return cudaErrorInvalidValue;
-    for (int j = 1; j < njobs; ++j)
-        if (jobs[j].g.rx != jobs[0].g.rx || jobs[j].g.ry != jobs[0].g.ry) {
-            if (ref) return cudaErrorInvalidValue;  // the per-reference pass runs one window size per launch
-            return launch_segments(jobs, njobs, tune, err, work, st);  // several window sizes
-        }
-    TcShape s;
-    if (!make_shape(jobs[0].g, tn, s)) return cudaErrorNotSupported;
-    std::unique_ptr<TcJobs> J(new TcJobs());
-    J->njobs = njobs;
+// All jobs of one window size (shape s under this tuning) in one launch.
+template <bool MULTI>
+cudaError_t launch_one_size(TcJobsT<MULTI ? kMaxTcJobs : 1>& J, const FftccJob* jobs, int njobs, const FftccTune& tune,
+                            TcShape s, unsigned* err, int* work, cudaStream_t st, bool ref, bool zeroed) {
+    J.njobs = njobs;
     int nb = 0;
     for (int j = 0; j < njobs; ++j) {
-        TcJob& o = J->job[j];
-        if (!fill_job(o, jobs[j], tn, s)) return cudaErrorInvalidValue;
+        TcJob& o = J.job[j];
+        if (!fill_job(o, jobs[j], tune, s)) return cudaErrorInvalidValue;
         o.batch_begin = nb;
         nb += (jobs[j].n + s.PB - 1) / s.PB;
     }
-    J->nbatch = nb;
+    J.nbatch = nb;
     if (nb == 0) return cudaSuccess;
     const uint4* tables = nullptr;
     {
@@ -1710,17 +1702,11 @@ cudaError_t launch_fftcc_tc_jobs(const FftccJob* jobs, int njobs, const FftccTun
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    void (*kern)(const TcJobs, TcShape, const uint4*, unsigned*, int*) = nullptr;
-    const bool multi = njobs > 1;
-#define TWDIC_TC_CASE(NPV, HPV)                                                                          \
-    case NPV * 100 + HPV:                                                                                \
-        if (ref)                                                                                         \
-            kern = multi ? k_fftcc_tc<NPV, HPV, true, false, true> : k_fftcc_tc<NPV, HPV, false, false, true>; \
-        else if (s.lo)                                                                                   \
-            kern = multi ? k_fftcc_tc<NPV, HPV, true, true, false> : k_fftcc_tc<NPV, HPV, false, true, false>; \
-        else                                                                                             \
-            kern = multi ? k_fftcc_tc<NPV, HPV, true, false, false>                                      \
-                         : k_fftcc_tc<NPV, HPV, false, false, false>;                                    \
+    void (*kern)(const TcJobsT<MULTI ? kMaxTcJobs : 1>, TcShape, const uint4*, unsigned*, int*) = nullptr;
+#define TWDIC_TC_CASE(NPV, HPV)                                                              \
+    case NPV * 100 + HPV:                                                                    \
+        kern = ref ? k_fftcc_tc<NPV, HPV, MULTI, false, true>                                \
+                   : (s.lo ? k_fftcc_tc<NPV, HPV, MULTI, true, false> : k_fftcc_tc<NPV, HPV, MULTI, false, false>); \
         break;
     switch (s.NP * 100 + s.HP) {
         TWDIC_TC_CASE(16, 8)
@@ -1752,18 +1738,44 @@ cudaError_t launch_fftcc_tc_jobs(const FftccJob* jobs, int njobs, const FftccTun
     int occ = 1;
     if (s.groups == 1 && 2 * (s.smem_bytes + 2048) <= 228 * 1024) occ = 2;
     const int grid = std::max(1, std::min(sms * occ, (nb + s.groups - 1) / s.groups));
-    e = cudaMemsetAsync(work, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
-    kern<<<grid, threads, s.smem_bytes, st>>>(*J, s, tables, err, work);
+    if (!zeroed) {
+        e = cudaMemsetAsync(work, 0, sizeof(int), st);
+        if (e != cudaSuccess) return e;
+    }
+    kern<<<grid, threads, s.smem_bytes, st>>>(J, s, tables, err, work);
     return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_fftcc_tc_jobs(const FftccJob* jobs, int njobs, const FftccTune& tune, unsigned* err, int* work,
+                                 cudaStream_t st, bool ref, bool zeroed) {
+    // the per-reference pass runs with single twiddles whatever the tuning
+    // (its spectra are rounded to FP16 when cached)
+    FftccTune tn = tune;
+    if (ref) tn.twiddle_lo = 0;
+    if (njobs < 1 || njobs > kMaxTcJobs) return cudaErrorInvalidValue;
+    for (int j = 1; j < njobs; ++j)
+        if (jobs[j].g.rx != jobs[0].g.rx || jobs[j].g.ry != jobs[0].g.ry) {
+            if (ref) return cudaErrorInvalidValue;  // the per-reference pass runs one window size per launch
+            return launch_segments(jobs, njobs, tune, err, work, st, zeroed);  // several window sizes
+        }
+    TcShape s;
+    if (!make_shape(jobs[0].g, tn, s)) return cudaErrorNotSupported;
+    if (njobs == 1) {
+        TcJobsT<1> one;
+        return launch_one_size<false>(one, jobs, njobs, tn, s, err, work, st, ref, zeroed);
+    }
+    std::unique_ptr<TcJobs> all(new TcJobs());
+    return launch_one_size<true>(*all, jobs, njobs, tn, s, err, work, st, ref, zeroed);
 }
 
 cudaError_t launch_fftcc_tc(const Geom& g, const uint8_t* ref_img, const uint8_t* tar_img, const void* maps,
                             uint64_t map_key, int uw, int utoff, uint32_t* fspec, int2* fsum, const int2* poi, int n, float* u, float* v, float* zncc, uint8_t* status,
-                            unsigned* err, int* work, const FftccTune& tune, cudaStream_t st, bool ref) {
+                            unsigned* err, int* work, const FftccTune& tune, cudaStream_t st, bool ref, bool zeroed) {
     if (n <= 0) return cudaSuccess;
     FftccJob job{g, maps, map_key, uw, utoff, ref_img, tar_img, fspec, fsum, poi, n, u, v, zncc, status};
-    return launch_fftcc_tc_jobs(&job, 1, tune, err, work, st, ref);
+    return launch_fftcc_tc_jobs(&job, 1, tune, err, work, st, ref, zeroed);
 }
 
 size_t fftcc_tc_spectrum_bytes(const Geom& g, int n) {

@@ -9,7 +9,7 @@
 // R_y dx, R_y dy) is formed per sample.
 //
 // Per target frame: the 4x4 byte neighbourhood of every ROI pixel (16 B,
-// k_nbhd_table), then one persistent kernel that runs the whole Gauss-Newton
+// k_prepare), then one persistent kernel that runs the whole Gauss-Newton
 // loop of each POI on chip.  Default layout (k_icgn_warp): one POI per warp,
 // the 32 warps of a CTA walking runs of consecutive POIs so that their
 // overlapping subsets are served from L1.  One-POI-per-CTA layout
@@ -245,62 +245,58 @@ __global__ void __launch_bounds__(kFactorThreads) k_ref_factor(int n, double* hi
     }
 }
 
-// 4x4 byte neighbourhood of every ROI pixel (i, j) of the target: rows
-// i-1 .. i+2, columns j-1 .. j+2 of the ROI-relative pixel, one 32-bit word
-// per row, lowest byte leftmost.  Bicubic (full = 0): zero on the ROI's last
-// row and column, the entries the reference's LUT never writes
+// The neighbourhood table: the 4x4 bytes around every ROI pixel (i, j) of the
+// target, rows i-1 .. i+2, columns j-1 .. j+2 of the ROI-relative pixel, one
+// 32-bit word per row, lowest byte leftmost.  Bicubic (full = 0): zero on the
+// ROI's last row and column, the entries the reference's LUT never writes
 // (TW_MemManager.cpp calloc).  The ROI has one pixel of border on every side
 // (validated on the host), and the neighbourhood of the other last-but-one
 // pixels stays inside the image.  B-spline (full = 1): every ROI pixel, with
 // the bytes outside the image zero, as the reference's B-spline LUT reads
 // them (TW_utils.cpp:521-602).
-__device__ __forceinline__ uint4 nbhd_entry(const Geom& g, const uint8_t* __restrict__ tar, int i, int j, int full) {
-    uint4 q = make_uint4(0u, 0u, 0u, 0u);
-    const int y0 = i + g.sy - 1, x0 = j + g.sx - 1;
-    if (!full && (i == g.rh - 1 || j == g.rw - 1)) {
-        // bicubic: the LUT's unwritten last row and column
-    } else if (y0 >= 0 && x0 >= 0 && y0 + 3 < g.img_h && x0 + 3 < g.img_w) {
-        const uint8_t* t = tar + (size_t)y0 * g.pitch + x0;
-        uint32_t w[4];
+//
+// kPrepRows entries of column j from row i0 down: each image row's four bytes
+// are read once (two aligned words and a funnel shift; the images carry 16
+// spare bytes) and serve the four entries they belong to, where one thread per
+// entry read 16 bytes one by one.  Bound by the 16 B written per entry.
+__device__ __forceinline__ void nbhd_column(const Geom& g, const uint8_t* __restrict__ tar, uint4* __restrict__ table,
+                                            int i0, int j, int full) {
+    const int x0 = j + g.sx - 1, y0 = i0 + g.sy - 1;  // at least 0: the ROI has a pixel of border
+    const int rows = min(kPrepRows, g.rh - i0);
+    const bool zero = !full && j == g.rw - 1;
+    // B-spline at the right edge: bytes outside the image are zero
+    const uint32_t mask = x0 + 4 <= g.img_w ? 0xffffffffu : 0xffffffffu >> (8 * (x0 + 4 - g.img_w));
+    const unsigned sh = 8u * (unsigned)(x0 & 3);
+    const uint8_t* src = tar + (size_t)y0 * g.pitch + (x0 & ~3);
+    uint32_t w[kPrepRows + 3];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const uint8_t* r = t + (size_t)a * g.pitch;
-            w[a] = (uint32_t)r[0] | ((uint32_t)r[1] << 8) | ((uint32_t)r[2] << 16) | ((uint32_t)r[3] << 24);
+    for (int a = 0; a < kPrepRows + 3; ++a) {
+        w[a] = 0u;
+        if (a < rows + 3 && y0 + a < g.img_h && !zero) {
+            const uint32_t* r = reinterpret_cast<const uint32_t*>(src + (size_t)a * g.pitch);
+            w[a] = __funnelshift_r(r[0], r[1], sh) & mask;
         }
-        q = make_uint4(w[0], w[1], w[2], w[3]);
-    } else {
-        // B-spline near the image edge: bytes outside the image are zero
-        uint32_t w[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            w[a] = 0u;
-            const int y = y0 + a;
-            if (y < 0 || y >= g.img_h) continue;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const int x = x0 + b;
-                if (x >= 0 && x < g.img_w) w[a] |= (uint32_t)tar[(size_t)y * g.pitch + x] << (8 * b);
-            }
-        }
-        q = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    return q;
+    uint4* out = table + (size_t)i0 * g.rw + j;
+#pragma unroll
+    for (int a = 0; a < kPrepRows; ++a) {
+        if (a >= rows) break;
+        const bool last = !full && i0 + a == g.rh - 1;  // bicubic: the LUT's unwritten last row
+        out[(size_t)a * g.rw] = last ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(w[a], w[a + 1], w[a + 2], w[a + 3]);
+    }
 }
 
-__global__ void k_nbhd_table(Geom g, const uint8_t* __restrict__ tar, uint4* __restrict__ table, int full) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= g.rh || j >= g.rw) return;
-    table[(size_t)i * g.rw + j] = nbhd_entry(g, tar, i, j, full);
-}
-
-// The per-frame preparation of a batch in one launch: the neighbourhood
-// tables of every frame that has one, then the zeroing of every frame's
-// output arrays that start at zero.  Items are numbered over all frames
-// (table pixels first, row-major per frame, then one item per POI); each
-// thread finds its frame by binary search over the frames' first items.
-__global__ void k_batch_prepare(const __grid_constant__ PrepJobs J) {
+// The per-frame preparation in one launch, of one frame or a batch: the
+// neighbourhood tables of the frames that have one, the zeroing of the output
+// arrays that start at zero, and the work counters of the launches that
+// follow.  Items are numbered over all frames (table items first, each a
+// column piece of kPrepRows entries, the columns of a piece side by side; then
+// one item per POI); each thread finds its frame by binary search over the
+// frames' first items.
+template <class Jobs>
+__global__ void k_prepare(const __grid_constant__ Jobs J) {
     const long long total = J.px_total + J.z_total;
+    if (blockIdx.x == 0 && (int)threadIdx.x < J.ncounters) J.counters[threadIdx.x] = 0;
     for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < total;
          k += (long long)gridDim.x * blockDim.x) {
         const bool px = k < J.px_total;
@@ -312,9 +308,9 @@ __global__ void k_batch_prepare(const __grid_constant__ PrepJobs J) {
         }
         const PrepJob& jb = J.job[lo];
         if (px) {
-            const long long o = item - jb.px_begin;
-            const int i = (int)(o / jb.g.rw), j = (int)(o - (long long)i * jb.g.rw);
-            jb.table[o] = nbhd_entry(jb.g, jb.tar, i, j, jb.full);
+            const unsigned o = (unsigned)(item - jb.px_begin);  // rw * ceil(rh / kPrepRows) items at most
+            const unsigned i = o / (unsigned)jb.g.rw;
+            nbhd_column(jb.g, jb.tar, jb.table, (int)i * kPrepRows, (int)(o - i * (unsigned)jb.g.rw), jb.full);
         } else {
             const long long p = item - jb.z_begin;
             for (int a = 0; a < 3; ++a)
@@ -608,14 +604,14 @@ __device__ __forceinline__ bool warp_end_pass(const IcgnJob& jb, int p, int it, 
 //   kSampLut: the per-frame bicubic coefficient LUT (four float4 planes,
 //     k_bicubic_lut), evaluated by Horner's rule;
 //   kSampNbhd: the per-frame 4x4 neighbourhood table (16 bytes per ROI
-//     pixel, k_nbhd_table), one 16-byte gather per sample, Catmull-Rom;
+//     pixel, k_prepare), one 16-byte gather per sample, Catmull-Rom;
 //   kSampNbhdBs: the same table over every ROI pixel, the reference's
 //     B-spline interpolant (bs_row_pair, bs_combine4x4).
 // The Catmull-Rom form with central-difference derivatives is algebraically
 // the reference's Hermite bicubic LUT (TW_utils.cpp:604-700).
 template <int THREADS, int SAMPLER, bool MULTI>
 __global__ void __launch_bounds__(THREADS, (THREADS == 64 ? 16 : 2048 / THREADS / 2))
-    k_icgn_fast(const __grid_constant__ IcgnJobs J, int* work) {
+    k_icgn_fast(const __grid_constant__ IcgnJobsT<MULTI ? kMaxJobs : 1> J, int* work) {
     constexpr int NW = THREADS / 32;
     constexpr unsigned FULL = 0xffffffffu;
     // dynamic shared memory: [S] half2 reference gradients (R_x, R_y: half
@@ -911,7 +907,7 @@ __global__ void k_ref_grad(Geom g, const uint8_t* __restrict__ ref, float2* __re
 // same sums, reduction, solve and update, so the results are identical.
 template <int NW, int SAMPLER, bool MULTI, int UNROLL>
 __global__ void __launch_bounds__(NW * 32, NW == 4 ? 4 : 32 / NW)
-    k_icgn_warp(const __grid_constant__ IcgnJobs J, int chunk) {
+    k_icgn_warp(const __grid_constant__ IcgnJobsT<MULTI ? kMaxJobs : 1> J, int chunk) {
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ int s_next;
     __shared__ WarpScratch s_sc[NW];
@@ -1060,7 +1056,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 4 : 32 / NW)
 // results are identical; warp 0 ends the pass.  It issues 2.3 times the
 // instructions of k_icgn_warp, so it is the faster one only on idle SMs.
 template <int NW, int SAMPLER, bool MULTI>
-__global__ void __launch_bounds__(NW * 32, 32 / NW) k_icgn_team(const __grid_constant__ IcgnJobs J) {
+__global__ void __launch_bounds__(NW * 32, 32 / NW) k_icgn_team(const __grid_constant__ IcgnJobsT<MULTI ? kMaxJobs : 1> J) {
     extern __shared__ __align__(16) float s_prod[];  // t', R_x t', R_y t' of the samples
     __shared__ WarpScratch sc;
     __shared__ float s_tot[8];
@@ -1176,27 +1172,22 @@ cudaError_t launch_ref_precompute_fast(const Geom& g, const uint8_t* ref, const 
     return cudaGetLastError();
 }
 
-cudaError_t launch_nbhd_table(const Geom& g, const uint8_t* tar, uint4* table, cudaStream_t st, bool full) {
-    dim3 blk(32, 8), grd((g.rw + 31) / 32, (g.rh + 7) / 8);
-    k_nbhd_table<<<grd, blk, 0, st>>>(g, tar, table, full ? 1 : 0);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_batch_prepare(const PrepJobs& J, cudaStream_t st) {
+template <class Jobs>
+static cudaError_t launch_prepare_t(const Jobs& J, cudaStream_t st) {
     const long long total = J.px_total + J.z_total;
-    if (total <= 0) return cudaSuccess;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long blocks = std::min<long long>((total + 255) / 256, (long long)sms * 8);
-    k_batch_prepare<<<(int)blocks, 256, 0, st>>>(J);
+    if (total <= 0 && J.ncounters <= 0) return cudaSuccess;
+    const long long blocks = std::max(1ll, std::min<long long>((total + 255) / 256, 1 << 20));
+    k_prepare<Jobs><<<(int)blocks, 256, 0, st>>>(J);
     return cudaGetLastError();
 }
+cudaError_t launch_prepare(const PrepJobs& J, cudaStream_t st) { return launch_prepare_t(J, st); }
+cudaError_t launch_prepare(const PrepJobsT<1>& J, cudaStream_t st) { return launch_prepare_t(J, st); }
 
 int icgn_fast_window(const Geom& g) { return 2 * (g.rx > g.ry ? g.rx : g.ry) + 1 + 10; }
 
 template <int THREADS, int SAMPLER, bool MULTI>
-static cudaError_t launch_icgn_fast_t(const IcgnJobs& J, int* work, int ctas_per_sm, cudaStream_t st) {
+static cudaError_t launch_icgn_fast_t(const IcgnJobsT<MULTI ? kMaxJobs : 1>& J, int* work, int ctas_per_sm,
+                                      cudaStream_t st) {
     int S_max = 0, ws_max = 0;
     for (int j = 0; j < J.njobs; ++j) {
         const Geom& g = J.job[j].g;
@@ -1262,7 +1253,8 @@ cudaError_t launch_ref_grad(const Geom& g, const uint8_t* ref, float2* grad, cud
 // by 10 (2048^2, 41x41 subsets: 2.27 ms against 2.31 ms by 8 or 6 and 2.25 ms
 // by 13, which loses 10 % on 61x61 subsets); CTAs of fewer warps: by 4.
 template <int NW, int SAMPLER, bool MULTI>
-static cudaError_t launch_icgn_warp_t(const IcgnJobs& J, int chunk, int ctas_per_sm, int unroll, cudaStream_t st) {
+static cudaError_t launch_icgn_warp_t(const IcgnJobsT<MULTI ? kMaxJobs : 1>& J, int chunk, int ctas_per_sm, int unroll,
+                                      cudaStream_t st) {
     auto kern = k_icgn_warp<NW, SAMPLER, MULTI, 4>;
     if (NW == 32 && unroll == 2) kern = k_icgn_warp<NW, SAMPLER, MULTI, (NW == 32 ? 2 : 4)>;
     if (NW == 32 && unroll == 8) kern = k_icgn_warp<NW, SAMPLER, MULTI, (NW == 32 ? 10 : 4)>;
@@ -1289,7 +1281,7 @@ static cudaError_t launch_icgn_warp_t(const IcgnJobs& J, int chunk, int ctas_per
 }
 
 template <int NW, int SAMPLER, bool MULTI>
-static cudaError_t launch_icgn_team_t(const IcgnJobs& J, cudaStream_t st) {
+static cudaError_t launch_icgn_team_t(const IcgnJobsT<MULTI ? kMaxJobs : 1>& J, cudaStream_t st) {
     int S = 0;
     for (int j = 0; j < J.njobs; ++j) S = std::max(S, (2 * J.job[j].g.rx + 1) * (2 * J.job[j].g.ry + 1));
     const int smem = 3 * S * (int)sizeof(float);
@@ -1303,7 +1295,8 @@ static cudaError_t launch_icgn_team_t(const IcgnJobs& J, cudaStream_t st) {
 // One POI per warp over a per-reference gradient image: every job needs
 // grad, the sample table, a table sampler and table offsets below 2^31
 // (otherwise the one-POI-per-CTA kernel runs).
-static bool icgn_warp_eligible(const IcgnJobs& J, const IcgnTune& tune) {
+template <class Jobs>
+static bool icgn_warp_eligible(const Jobs& J, const IcgnTune& tune) {
     if (tune.chunk <= 0 || tune.sampler == kSampWindow) return false;
     if (tune.threads != 128 && tune.threads != 256 && tune.threads != 512 && tune.threads != 1024) return false;
     for (int j = 0; j < J.njobs; ++j) {
@@ -1314,16 +1307,14 @@ static bool icgn_warp_eligible(const IcgnJobs& J, const IcgnTune& tune) {
     return true;
 }
 
-cudaError_t launch_icgn_fast_jobs(const IcgnJobs& J, int* work, const IcgnTune& tune, cudaStream_t st) {
-    if (J.njobs < 1 || J.njobs > kMaxJobs) return cudaErrorInvalidValue;
-    if (J.total <= 0) return cudaSuccess;
+template <bool MULTI>
+static cudaError_t launch_icgn_jobs(const IcgnJobsT<MULTI ? kMaxJobs : 1>& J, int* work, const IcgnTune& tune,
+                                    cudaStream_t st) {
     if (icgn_warp_eligible(J, tune)) {
         for (int j = 0; j < J.njobs; ++j)
             if (!J.job[j].table) return cudaErrorInvalidValue;
-        const bool multi = J.njobs > 1;
 #define TWDIC_ICGN_WARP(NW, SA)                                                                  \
-    return multi ? launch_icgn_warp_t<NW, SA, true>(J, tune.chunk, tune.ctas_per_sm, tune.unroll, st)  \
-                 : launch_icgn_warp_t<NW, SA, false>(J, tune.chunk, tune.ctas_per_sm, tune.unroll, st)
+    return launch_icgn_warp_t<NW, SA, MULTI>(J, tune.chunk, tune.ctas_per_sm, tune.unroll, st)
 #define TWDIC_ICGN_WARP_N(NW)                                                                    \
     if (tune.sampler == kSampLut) { TWDIC_ICGN_WARP(NW, kSampLut); }                              \
     if (tune.sampler == kSampNbhdBs) { TWDIC_ICGN_WARP(NW, kSampNbhdBs); }                        \
@@ -1340,7 +1331,7 @@ cudaError_t launch_icgn_fast_jobs(const IcgnJobs& J, int* work, const IcgnTune& 
         const bool full = tune.threads == 1024 && tune.sampler != kSampLut;
         if (full && J.total <= 4 * sms) {
 #define TWDIC_ICGN_TEAM(SA)                                                                                \
-    return multi ? launch_icgn_team_t<8, SA, true>(J, st) : launch_icgn_team_t<8, SA, false>(J, st)
+    return launch_icgn_team_t<8, SA, MULTI>(J, st)
             if (tune.sampler == kSampNbhdBs) { TWDIC_ICGN_TEAM(kSampNbhdBs); }
             TWDIC_ICGN_TEAM(kSampNbhd);
 #undef TWDIC_ICGN_TEAM
@@ -1360,10 +1351,8 @@ cudaError_t launch_icgn_fast_jobs(const IcgnJobs& J, int* work, const IcgnTune& 
         return cudaErrorInvalidValue;
     for (int j = 0; j < J.njobs; ++j)
         if (t1.sampler != kSampWindow && !J.job[j].table) return cudaErrorInvalidValue;
-    const bool multi = J.njobs > 1;
 #define TWDIC_ICGN_FAST(TH, SA)                                                                  \
-    return multi ? launch_icgn_fast_t<TH, SA, true>(J, work, t1.ctas_per_sm, st)               \
-                 : launch_icgn_fast_t<TH, SA, false>(J, work, t1.ctas_per_sm, st)
+    return launch_icgn_fast_t<TH, SA, MULTI>(J, work, t1.ctas_per_sm, st)
 #define TWDIC_ICGN_FAST_T(TH)                                                                    \
     if (t1.sampler == kSampLut) { TWDIC_ICGN_FAST(TH, kSampLut); }                              \
     if (t1.sampler == kSampNbhd) { TWDIC_ICGN_FAST(TH, kSampNbhd); }                            \
@@ -1377,13 +1366,24 @@ cudaError_t launch_icgn_fast_jobs(const IcgnJobs& J, int* work, const IcgnTune& 
 #undef TWDIC_ICGN_FAST
 }
 
+cudaError_t launch_icgn_fast_jobs(const IcgnJobs& J, int* work, const IcgnTune& tune, cudaStream_t st) {
+    if (J.njobs < 1 || J.njobs > kMaxJobs) return cudaErrorInvalidValue;
+    if (J.total <= 0) return cudaSuccess;
+    if (J.njobs > 1) return launch_icgn_jobs<true>(J, work, tune, st);
+    IcgnJobsT<1> one;
+    one.njobs = 1;
+    one.total = J.total;
+    one.job[0] = J.job[0];
+    return launch_icgn_jobs<false>(one, work, tune, st);
+}
+
 cudaError_t launch_icgn_fast(const Geom& g, const uint8_t* ref, const uint8_t* tar, const int2* poi, int n,
                              const float* stats, const double* chol, const uint8_t* rflag, const void* table,
                              int* work, float* u, float* v, float* p6, int* iters, uint8_t* flags,
                              const IcgnTune& tune, cudaStream_t st, const float2* grad,
                              const float4* samples) {
     if (n <= 0) return cudaSuccess;
-    IcgnJobs J;
+    IcgnJobsT<1> J;
     J.njobs = 1;
     J.total = n;
     IcgnJob& jb = J.job[0];
@@ -1404,7 +1404,7 @@ cudaError_t launch_icgn_fast(const Geom& g, const uint8_t* ref, const uint8_t* t
     jb.flags = flags;
     jb.n = n;
     jb.begin = 0;
-    return launch_icgn_fast_jobs(J, work, tune, st);
+    return launch_icgn_jobs<false>(J, work, tune, st);
 }
 
 }  // namespace twdic
