@@ -450,6 +450,34 @@ __device__ __forceinline__ void cr_weights(float t, float& w0, float& w1, float&
     w3 = t2 * (0.5f * t - 0.5f);
 }
 
+// f(smp + k) for the samples k = lane + 32 j < S of a warp in order, smp their
+// table from the lane's first entry on: blocks of UNROLL steps (2, 4 or 8), then
+// shorter ones, then the steps that are left, the last with the lanes that have
+// a sample.  The trip counts are the warp's, not the lane's: a loop over k < S
+// unrolled by the compiler ran its last block for some lanes and its remainder
+// for the others (25x25 subsets, 19.5 steps: 364 us against 260 us; 41x41: 2.28
+// against 2.23 ms).
+template <int N, class F>
+__device__ __forceinline__ void sample_steps(const float4* smp, const F& f) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) f(smp + 32 * j);
+}
+template <int UNROLL, class F>
+__device__ __forceinline__ void for_samples(const float4* smp, int S, const F& f) {
+    const int lane = threadIdx.x & 31;
+    int left = S;
+    for (; left >= 32 * UNROLL; left -= 32 * UNROLL, smp += 32 * UNROLL) sample_steps<UNROLL>(smp, f);
+    if (UNROLL > 4 && left >= 128) {
+        sample_steps<4>(smp, f);
+        left -= 128;
+        smp += 128;
+    }
+    for (; UNROLL > 2 && left >= 64; left -= 64, smp += 64) sample_steps<2>(smp, f);
+#pragma unroll 1
+    for (; left > 0; left -= 32, smp += 32)
+        if (lane < left) f(smp);
+}
+
 // Affine warp of subset offset (dx, dy) as two FMAs per coordinate.  The
 // reference rounds each operation; the difference is an ulp, which moves a
 // truncated coordinate only at an exact integer, where the bicubic patch is
@@ -979,13 +1007,11 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 4 : 32 / NW)
                     // from a whole-pixel guess: the subset of the image shifted
                     // by it, no coordinates
                     const uint8_t* t0 = jb.tar + ((size_t)((int)by - g.ry) * g.pitch + ((int)bx - g.rx));
-#pragma unroll UNROLL
-                    for (int k = lane; k < S; k += 32) {
-                        const float4 e4 = __ldg(smp);
-                        smp += 32;
+                    for_samples<UNROLL>(smp0, S, [&](const float4* sp) {
+                        const float4 e4 = __ldg(sp);
                         const int ox = __float_as_int(e4.z), oy = __float_as_int(e4.w);
                         ps.add((float)t0[oy * g.pitch + ox] - c, grad0[oy * g.rw + ox], make_float2(e4.x, e4.y));
-                    }
+                    });
                 } else if (it == 0) {
                     // first pass from a fractional guess: truncated coordinates
 #pragma unroll 2
@@ -1000,10 +1026,8 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 4 : 32 / NW)
                         ps.add((float)jb.tar[(size_t)iy * g.pitch + ix] - c, grad0[gofs], d);
                     }
                 } else {
-#pragma unroll UNROLL
-                    for (int k = lane; k < S; k += 32) {
-                        const float4 e4 = __ldg(smp);
-                        smp += 32;
+                    for_samples<UNROLL>(smp0, S, [&](const float4* sp) {
+                        const float4 e4 = __ldg(sp);
                         const float2 d = make_float2(e4.x, e4.y);
                         const int gofs = __float_as_int(e4.w) * g.rw + __float_as_int(e4.z);
                         const float2 wxy = __ffma2_rn(w03, make_float2(d.x, d.x),
@@ -1035,7 +1059,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 4 ? 4 : 32 / NW)
                             tp = (((r23.y * fy + r23.x) * fy + r01.y) * fy + r01.x) - c;
                         }
                         ps.add(tp, grad0[gofs], d);
-                    }
+                    });
                 }
                 ps.unpack(s);
                 v8 = warp_reduce8(s);
@@ -1249,15 +1273,15 @@ cudaError_t launch_ref_grad(const Geom& g, const uint8_t* ref, float2* grad, cud
     return cudaGetLastError();
 }
 
-// unroll: the sample loops' unrolling, 2, 4 or, as "8", the deepest, which is
-// by 10 (2048^2, 41x41 subsets: 2.27 ms against 2.31 ms by 8 or 6 and 2.25 ms
-// by 13, which loses 10 % on 61x61 subsets); CTAs of fewer warps: by 4.
+// unroll: the sample loops' blocks, 2, 4 or 8 steps for the one-CTA-per-SM shape
+// (2048^2, 41x41 subsets: 2.23 ms by 8, 2.24 by 6, 2.23 by 10, 2.27 by 16), 4 for
+// CTAs of fewer warps.
 template <int NW, int SAMPLER, bool MULTI>
 static cudaError_t launch_icgn_warp_t(const IcgnJobsT<MULTI ? kMaxJobs : 1>& J, int chunk, int ctas_per_sm, int unroll,
                                       cudaStream_t st) {
     auto kern = k_icgn_warp<NW, SAMPLER, MULTI, 4>;
     if (NW == 32 && unroll == 2) kern = k_icgn_warp<NW, SAMPLER, MULTI, (NW == 32 ? 2 : 4)>;
-    if (NW == 32 && unroll == 8) kern = k_icgn_warp<NW, SAMPLER, MULTI, (NW == 32 ? 10 : 4)>;
+    if (NW == 32 && unroll == 8) kern = k_icgn_warp<NW, SAMPLER, MULTI, (NW == 32 ? 8 : 4)>;
     // shared memory for the resident CTAs (up to 8 KB each with the runtime's
     // 1 KB; at a share of 0 the smaller CTAs are not all resident), the rest of
     // the SM's 256 KB to L1
