@@ -55,7 +55,9 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kCandChunk = 128;   // exact re-evaluations per pass (all POIs of a group batch)
-constexpr int kMaxPB = 8;         // POIs per batch (upper bound)
+// POIs per batch (upper bound) by HP: the small windows fill the 128 rows of
+// stages 2 and 3 with more than eight POIs (14 of 16x16, 9 of 24x24)
+constexpr int max_pb(int hp) { return hp <= 16 ? 16 : 8; }
 constexpr int kMaxGroups = 5;     // 128-thread groups per CTA (upper bound; window sizes up to 48)
 constexpr int kSegGroups = 4;     // groups per CTA of the larger windows and of the segmented kernel
 // Candidate window of the approximate correlation surface, in ZNCC units.
@@ -82,6 +84,7 @@ struct TcShape {
     int tcols;      // TMEM columns per group (96 or 128): the widest accumulator of the four stages
     int uw, utoff;  // one-row boxes: width (0: none for this geometry) and the target box's offset
     int win_bytes;  // a group's window region
+    int cta_bytes;  // the CTA's shared state, before the tables
     int tiles4;  // 128-row tiles of the surface (stage 4)
     int FS;      // complex values per cached spectrum row: N rounded up to 4
     int NW4;  // 32-bit words per window row in the exact re-evaluation
@@ -317,28 +320,35 @@ __device__ __forceinline__ void st_half(uint8_t* p, float v) { *reinterpret_cast
 // share one region: each is written only after the MMA that reads the
 // previous one has completed.
 
-// Shared state of a CTA's groups (static shared memory).
-struct TcCta {
+// Shared state of a CTA's groups, at the start of its dynamic shared memory
+// (its size goes by the window size; the segmented kernel changes it between
+// segments, the head stays).
+struct TcHead {
     uint64_t mbar_mma[kMaxGroups];
     uint64_t mbar_tma[kMaxGroups][2];  // one per window slot
     uint32_t tmem_slot;
     int seg;
-    int wsum[kMaxGroups][2 * kMaxPB][2];
-    float sscale[kMaxGroups][kMaxPB];
-    int sdark[kMaxGroups][kMaxPB];
-    int cbase[kMaxGroups][kMaxPB];      // first candidate slot of each POI
-    int cend[kMaxGroups][kMaxPB];       // one past its last
-    int wtot[kMaxGroups][2][4];         // candidates per warp and surface tile
-    uint32_t smaxv[kMaxGroups][kMaxPB];  // ordered value of the approximate peak
+    int snext[kMaxGroups];
+};
+template <int PBM>
+struct TcCta : TcHead {
+    int wsum[kMaxGroups][2 * PBM][2];
+    float sscale[kMaxGroups][PBM];
+    int sdark[kMaxGroups][PBM];
+    int cbase[kMaxGroups][PBM];      // first candidate slot of each POI
+    int cend[kMaxGroups][PBM];       // one past its last
+    int wtot[kMaxGroups][2][4];      // candidates per warp and surface tile
+    uint32_t smaxv[kMaxGroups][PBM];  // ordered value of the approximate peak
     // per window slot (a group's batch in work and the next one, staged
     // while the first runs): POIs, each window's (0, 0) (staged box or the
     // image), the windows' row stride, 1 when they are the staged boxes
-    int2 spoi[kMaxGroups][2][kMaxPB];
-    const uint8_t* wptr[kMaxGroups][2][2 * kMaxPB];
+    int2 spoi[kMaxGroups][2][PBM];
+    const uint8_t* wptr[kMaxGroups][2][2 * PBM];
     int wrs[kMaxGroups][2];
     int wsm[kMaxGroups][2];
-    int snext[kMaxGroups];
 };
+template <int PBM>
+constexpr int kCtaBytes = ((int)sizeof(TcCta<PBM>) + 1023) / 1024 * 1024;
 
 // The tensor maps of jobs [lo, hi): visible to the tensor-map proxy (they
 // were written to device memory by copies) and prefetched.  Thread 0 of each
@@ -391,14 +401,16 @@ __device__ __forceinline__ void zero_a4_padding(uint8_t* a4, const TcShape& s, i
 template <int NP, int HP, bool MULTI, bool LO, bool REF, class Jobs>
 __device__ __forceinline__ bool tc_group_batches(const Jobs& J, const TcShape& s, int job_lo, int job_hi,
                                                  int nbatch, int first, int* counter, int counter_base,
-                                                 unsigned* err, TcCta& cs, uint8_t* sm, uint32_t& phase,
+                                                 unsigned* err, uint8_t* sm0, uint32_t& phase,
                                                  uint32_t& tphase) {
     const int grp = threadIdx.x >> 7;
     const int t = threadIdx.x & 127, warp = t >> 5, lane = t & 31;
     const int bar_id = 1 + grp;
     const int N = s.N, H = s.H, PB = s.PB, K4 = s.K4;
     const int n2 = N * N;
-    constexpr int K1 = NP;
+    constexpr int K1 = NP, PBM = max_pb(HP);
+    TcCta<PBM>& cs = *reinterpret_cast<TcCta<PBM>*>(sm0);
+    uint8_t* sm = sm0 + kCtaBytes<PBM>;
     uint8_t* gbase = sm + s.tab_bytes + grp * s.group_bytes;
     // window slots 0 and 1, win_bytes apart: the two one-row TMA boxes,
     // reference at 0, target at utoff
@@ -515,7 +527,7 @@ __device__ __forceinline__ bool tc_group_batches(const Jobs& J, const TcShape& s
             if (!REF && b0 + t < n_job) fsum = jb.fsum[b0 + t];
         }
         if (t == 0) nxt = have_next ? counter_base + atomicAdd(counter, 1) : nbatch;  // the batch after nb
-        if (t < 2 * kMaxPB * 2) (&cs.wsum[grp][0][0])[t] = 0;
+        if (t < 2 * PBM * 2) (&cs.wsum[grp][0][0])[t] = 0;
         if (t < PB) cs.smaxv[grp][t] = 0u;
         // this batch's windows (staged one batch earlier)
         // (each wait below: the threads agree that none gave up at the next
@@ -1194,7 +1206,7 @@ __device__ __forceinline__ bool tc_group_batches(const Jobs& J, const TcShape& s
 // TMEM columns and mbarriers of the CTA's groups; false (err set, TMEM
 // freed) when the dynamic shared memory is not 128-byte aligned, which the
 // TMA destinations need.  Ends with a CTA barrier.
-__device__ __forceinline__ bool tc_setup(TcCta& cs, uint8_t* sm, int groups, uint32_t tmem_cols, unsigned* err) {
+__device__ __forceinline__ bool tc_setup(TcHead& cs, uint8_t* sm, int groups, uint32_t tmem_cols, unsigned* err) {
     if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(&cs.tmem_slot)),
@@ -1221,7 +1233,7 @@ __device__ __forceinline__ bool tc_setup(TcCta& cs, uint8_t* sm, int groups, uin
     return true;
 }
 
-__device__ __forceinline__ void tc_teardown(TcCta& cs, uint32_t tmem_cols) {
+__device__ __forceinline__ void tc_teardown(TcHead& cs, uint32_t tmem_cols) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1238,16 +1250,16 @@ __global__ void __launch_bounds__(NP <= 48 ? 128 * kMaxGroups : 128 * kSegGroups
                                                                  const uint4* __restrict__ tables, unsigned* err,
                                                                  int* work) {
     extern __shared__ __align__(1024) uint8_t sm[];
-    __shared__ TcCta cs;
+    TcHead& cs = *reinterpret_cast<TcHead*>(sm);
     const int grp = threadIdx.x >> 7;
     uint32_t tmem_cols = 32u;  // the groups' columns, allocated as a power of two
     while (tmem_cols < (uint32_t)(s.groups * s.tcols)) tmem_cols <<= 1;
-    tc_load_tables(sm, tables, s.tab_bytes);
+    tc_load_tables(sm + kCtaBytes<max_pb(HP)>, tables, s.tab_bytes);
     if ((threadIdx.x & 127) == 0) tc_acquire_maps(J, 0, J.njobs);
     if (!tc_setup(cs, sm, s.groups, tmem_cols, err)) return;
     uint32_t phase = 0, tphase = 0;
     tc_group_batches<NP, HP, MULTI, LO, REF>(J, s, 0, J.njobs, J.nbatch, blockIdx.x * s.groups + grp, work,
-                                        gridDim.x * s.groups, err, cs, sm, phase, tphase);
+                                        gridDim.x * s.groups, err, sm, phase, tphase);
     tc_teardown(cs, tmem_cols);
 }
 
@@ -1257,7 +1269,7 @@ constexpr int kTcShapes[8][2] = {{16, 8}, {16, 16}, {32, 16}, {32, 24}, {48, 24}
 
 template <bool LO>
 __device__ __forceinline__ bool tc_run_segment(const TcJobs& J, const TcSeg& sg, int* counter, unsigned* err,
-                                               TcCta& cs, uint8_t* sm, uint32_t& phase, uint32_t& tphase) {
+                                               TcHead& cs, uint8_t* sm, uint32_t& phase, uint32_t& tphase) {
     const int grp = threadIdx.x >> 7;
     if (grp >= sg.s.groups) return true;  // this segment's shared memory holds fewer groups
     // every batch, the first included, from the segment's counter
@@ -1268,7 +1280,7 @@ __device__ __forceinline__ bool tc_run_segment(const TcJobs& J, const TcSeg& sg,
     case K:                                                                                                  \
         return tc_group_batches<kTcShapes[K][0], kTcShapes[K][1], true, LO, false>(J, sg.s, sg.job_lo,       \
                                                                             sg.job_hi, sg.nbatch, first,     \
-                                                                            counter, 0, err, cs, sm, phase,  \
+                                                                            counter, 0, err, sm, phase,      \
                                                                             tphase);
     switch (sg.shape) {
         TWDIC_TC_SEG(0)
@@ -1296,7 +1308,7 @@ __global__ void __launch_bounds__(128 * kSegGroups, 1) k_fftcc_tc_seg(const __gr
                                                                      const __grid_constant__ TcSegs S,
                                                                      unsigned* err, int* counters) {
     extern __shared__ __align__(1024) uint8_t sm[];
-    __shared__ TcCta cs;
+    TcHead& cs = *reinterpret_cast<TcHead*>(sm);
     constexpr uint32_t tmem_cols = 512u;
     if (!tc_setup(cs, sm, kSegGroups, tmem_cols, err)) return;
     if ((threadIdx.x & 127) == 0) tc_acquire_maps(J, 0, J.njobs);
@@ -1305,7 +1317,7 @@ __global__ void __launch_bounds__(128 * kSegGroups, 1) k_fftcc_tc_seg(const __gr
     uint32_t phase = 0, tphase = 0;
     for (;;) {
         const TcSeg& sg = S.seg[seg];
-        tc_load_tables(sm, sg.tables, sg.s.tab_bytes);
+        tc_load_tables(sm + sg.s.cta_bytes, sg.tables, sg.s.tab_bytes);
         __syncthreads();
         const bool ok = tc_run_segment<LO>(J, sg, counters + seg, err, cs, sm, phase, tphase);
         // every group is done with this segment's tables; the next segment
@@ -1344,7 +1356,9 @@ bool make_shape(const Geom& g, const FftccTune& tune, TcShape& s) {
     // POIs per batch: the (POI, ky) rows of stages 2 and 3 fill one 128-row
     // tile; the (POI, x) rows of stages 1 and 4 take up to two, each with its
     // own TMEM columns (2 HP at stage 1, NP at stage 4) within the group's 128
-    int pb = std::min(128 / s.H, kMaxPB);
+    int pb = std::min(128 / s.H, max_pb(s.HP));
+    // beyond eight only as long as one box holds the batch's windows
+    if (g.grid_x > 0) pb = std::min(pb, std::max(8, (256 - 15 - N) / g.grid_x + 1));
     if (tune.pois_per_group > 0) pb = std::min(pb, tune.pois_per_group);  // tuned batch size
     int tiles = 0;
     for (; pb >= 1; --pb) {
@@ -1415,8 +1429,9 @@ bool make_shape(const Geom& g, const FftccTune& tune, TcShape& s) {
     s.win_bytes = round_up(s.utoff + N * s.uw + 16, 128);
     s.off_win = region;
     s.group_bytes = round_up(region + 2 * s.win_bytes, 1024);  // two window slots
-    // 227 KB per CTA, less the static state (the dynamic part starts 1024-byte aligned)
-    const int limit = 227 * 1024 - round_up((int)sizeof(TcCta), 1024);
+    // 227 KB per CTA, less the groups' state
+    s.cta_bytes = max_pb(s.HP) == 16 ? kCtaBytes<16> : kCtaBytes<8>;
+    const int limit = 227 * 1024 - s.cta_bytes;
     // TMEM: each group's widest accumulator (stage 1: tiles x 2 HP, stages 2
     // and 3: 2 NP, stage 4: tiles x NP), 96 columns up to N = 48, so five
     // groups share the 512 columns there, four above
@@ -1424,8 +1439,8 @@ bool make_shape(const Geom& g, const FftccTune& tune, TcShape& s) {
     s.groups = std::min(std::min(kMaxGroups, 512 / s.tcols), (limit - o) / s.group_bytes);
     if (tune.groups > 0) s.groups = std::min(s.groups, tune.groups);  // tuned group count
     if (s.groups < 1) return false;
-    s.smem_bytes = o + s.groups * s.group_bytes;
-    return s.smem_bytes <= limit;
+    s.smem_bytes = s.cta_bytes + o + s.groups * s.group_bytes;
+    return s.smem_bytes <= 227 * 1024;
 }
 
 // Twiddle matrices B1, C2, S2, B4 (hi and lo FP16) in the no-swizzle K-major
