@@ -166,6 +166,9 @@ struct Engine {
     // launch shape changes
     DevBuf d_tcmaps;
     void* h_tcmaps = nullptr;
+    // pinned words beside them that calls read back (an asynchronous copy into
+    // pageable memory would be staged): [0] error flags, [1] POIs changed
+    volatile unsigned* h_words = nullptr;
     TcMapInfo tcmaps{0, 0, 0};
     // per-reference cache of the tensor-core FFT-CC: the reference windows'
     // spectra and integer sums at the POIs (dropped with the IC-GN cache)
@@ -215,7 +218,8 @@ struct Engine {
         TW_TRY(d_err.ensure(sizeof(unsigned)));
         TW_TRY(d_work.ensure(sizeof(int) * 4));
         TW_TRY(d_tcmaps.ensure(kTcMapsBytes));
-        TW_CUDA(cudaMallocHost(&h_tcmaps, kTcMapsBytes));
+        TW_CUDA(cudaMallocHost(&h_tcmaps, kTcMapsBytes + 2 * sizeof(unsigned)));
+        h_words = reinterpret_cast<unsigned*>(static_cast<char*>(h_tcmaps) + kTcMapsBytes);
         TW_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(unsigned), stream));
         // DFT twiddles exp(-2 pi i k / N) of the two window sizes, rounded once
         // from double (the FP32 SIMT FFT-CC kernel reads them)
@@ -259,10 +263,10 @@ struct Engine {
     }
 
     int check_err() {
-        unsigned h = 0;
-        TW_CUDA(cudaMemcpyAsync(&h, d_err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
+        TW_CUDA(cudaMemcpyAsync(const_cast<unsigned*>(h_words), d_err.p, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                                stream));
         TW_CUDA(cudaStreamSynchronize(stream));
-        if (h & kErrTimeout) {
+        if (h_words[0] & kErrTimeout) {
             cudaMemsetAsync(d_err.p, 0, sizeof(unsigned), stream);
             return fail(TWDIC_ERR_TIMEOUT, "a bounded device-side wait gave up");
         }
@@ -376,12 +380,6 @@ struct Engine {
         cache_valid = true;
         if (t_pre) *t_pre = 1.f;
         return TWDIC_OK;
-    }
-
-    // IC-GN of all POIs; u, v in/out device arrays.
-    int icgn(float* u, float* v, float* p6, int* iters, uint8_t* flags) {
-        TW_TRY(prepare_target());
-        return icgn_solve(u, v, p6, iters, flags);
     }
 
     // Per-target preparation: the table the IC-GN variant reads, the bicubic
@@ -600,31 +598,38 @@ int twdic_icgn_compute(twdic_icgn* h, const uint8_t* tar, int32_t stride, const 
     TW_TRY(check_mem(mem_out));
     Engine& e = h->e;
     const size_t n = (size_t)e.n;
-    TW_TRY(e.set_tar(tar, stride, mem_in));
     // POIs: the per-reference cache is keyed on their contents.  Host POIs
     // are compared with a host copy; device POIs are copied into the handle's
     // array on every call by a kernel that reports whether any pair changed
     // (the caller may rewrite the same buffer, or an allocator may hand its
-    // address to new POIs).
+    // address to new POIs).  The host waits for that answer while the target's
+    // copy and table, which do not depend on it, run.
     if (mem_in == TWDIC_MEM_HOST) {
+        TW_TRY(e.set_tar(tar, stride, mem_in));
         if (e.cache_poi_host.size() != 2 * n || std::memcmp(e.cache_poi_host.data(), poi_yx, 8 * n) != 0) {
             e.cache_poi_host.assign(poi_yx, poi_yx + 2 * n);
             TW_TRY(copy_in(e.d_poi.p, poi_yx, 8 * n, mem_in, e.stream));
             e.cache_valid = false;
             e.fspec_valid = false;
         }
+        TW_TRY(e.prepare_target());
     } else {
         int* changed_d = e.d_work.as<int>() + 2;
-        int changed = 0;
         TW_CUDA(cudaMemsetAsync(changed_d, 0, sizeof(int), e.stream));
         TW_CUDA(launch_poi_refresh(poi_yx, e.d_poi.as<int2>(), (int)n, changed_d, e.stream));
-        TW_CUDA(cudaMemcpyAsync(&changed, changed_d, sizeof(int), cudaMemcpyDeviceToHost, e.stream));
-        TW_CUDA(cudaStreamSynchronize(e.stream));
-        if (changed) {
+        TW_CUDA(cudaMemcpyAsync(const_cast<unsigned*>(e.h_words + 1), changed_d, sizeof(int), cudaMemcpyDeviceToHost,
+                                e.stream));
+        TW_CUDA(cudaEventRecord(e.ev_sync, e.stream));
+        int rc = e.set_tar(tar, stride, mem_in);
+        if (rc == TWDIC_OK) rc = e.prepare_target();
+        const cudaError_t waited = cudaEventSynchronize(e.ev_sync);
+        if (waited != cudaSuccess || e.h_words[1]) {
             e.cache_poi_host.clear();
             e.cache_valid = false;
             e.fspec_valid = false;
         }
+        TW_TRY(rc);
+        TW_CUDA(waited);
     }
     float *du = u, *dv = v, *dp6 = p6 ? p6 : e.d_p6.as<float>();
     int* dit = iters;
@@ -640,7 +645,7 @@ int twdic_icgn_compute(twdic_icgn* h, const uint8_t* tar, int32_t stride, const 
         dit = e.d_iters.as<int>();
         TW_CUDA(cudaMemsetAsync(dit, 0, 4 * n, e.stream));
     }
-    TW_TRY(e.icgn(du, dv, dp6, dit, dfl));
+    TW_TRY(e.icgn_solve(du, dv, dp6, dit, dfl));
     if (mem_out == TWDIC_MEM_HOST) {
         TW_TRY(copy_out(u, du, 4 * n, mem_out, e.stream));
         TW_TRY(copy_out(v, dv, 4 * n, mem_out, e.stream));
