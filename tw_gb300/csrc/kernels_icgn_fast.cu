@@ -1310,7 +1310,11 @@ static cudaError_t launch_icgn_team_t(const IcgnJobsT<MULTI ? kMaxJobs : 1>& J, 
     for (int j = 0; j < J.njobs; ++j) S = std::max(S, (2 * J.job[j].g.rx + 1) * (2 * J.job[j].g.ry + 1));
     const int smem = 3 * S * (int)sizeof(float);
     auto kern = k_icgn_team<NW, SAMPLER, MULTI>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // one value for every subset (radii up to 31): another thread's launch of
+    // smaller subsets never lowers the limit between this call and the launch
+    constexpr int kMaxSmem = 3 * 63 * 63 * (int)sizeof(float);
+    if (smem > kMaxSmem) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e != cudaSuccess) return e;
     kern<<<J.total, NW * 32, smem, st>>>(J);
     return cudaGetLastError();
