@@ -397,7 +397,7 @@ def _run_gpu(args, world, rank, local, torch):
             "e2e": {"value": round(e2e_value, 1), "unit": UNIT, "h2d_bytes_per_step": int(pair.tar.nbytes),
                     "d2h_bytes_per_step": d2h, "p50_ms": round(pct(e2e_ms, 50), 4),
                     "p99_ms": round(pct(e2e_ms, 99), 4)},
-            # per frame: k_fftcc_tc, k_nbhd_table, k_icgn_warp
+            # per frame: k_prepare, k_fftcc_tc, k_icgn_warp
             "gpu_launches": 3 * args.steps,
             "clocks": clk,
             "wall_s_timed_region": round(t_wall, 3)}
@@ -454,11 +454,11 @@ def _run_gpu(args, world, rank, local, torch):
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of one launch
 # of each kernel on this workload, from the ncu captures summarised in
 # profiles/k_icgn_warp_2048_subset41.md and profiles/k_fftcc_tc_2048_subset41.md
-NCU_TRAFFIC = {"k_icgn_warp": 139.83e6 + 7.27e6, "k_fftcc_tc": 532.76e6 + 5.50e6}
+NCU_TRAFFIC = {"k_icgn_warp": 139.78e6 + 7.98e6, "k_fftcc_tc": 532.43e6 + 5.24e6}
 # from the same IC-GN capture: L1 hit rate of its gathers and the FMA-heavy
 # pipe's share of cycles (the kernel's limiter)
-NCU_ICGN_L1_HIT = 0.933
-NCU_ICGN_FMAHEAVY = 0.667
+NCU_ICGN_L1_HIT = 0.929
+NCU_ICGN_FMAHEAVY = 0.680
 
 
 def fp32_peak(peaks):
@@ -481,8 +481,8 @@ def roofline(g, P, ph, kbar):
     the per-phase CUDA events of the frame.
 
     Binding view (bound / achieved / peak / frac): FP32.  The kernel is
-    limited by the SM's FP32 and integer pipes (ncu: FMA-heavy pipe busy 67 %
-    of cycles, 77 % issue) with its gathers served by L1 (93 % hits); the
+    limited by the SM's FP32 and integer pipes (ncu: FMA-heavy pipe busy 68 %
+    of cycles, 75 % issue) with its gathers served by L1 (93 % hits); the
     credited work is k*S*64 flops per POI (k = mean iterations, S = subset
     pixels; 64 flops per sample and iteration: warp 8, bicubic Horner 30,
     mean/norm 6, residual 4, right-hand side 12, address 4), against the

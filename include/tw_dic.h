@@ -175,7 +175,8 @@ TWDIC_API int twdic_frame_process(twdic_frame* h, const uint8_t* tar, int32_t st
  * handle's own stream).  All work of later calls is ordered on it. */
 TWDIC_API int twdic_frame_set_stream(twdic_frame* h, void* stream);
 /* Device time of the phases of the last process call, in milliseconds:
- * t[0] target upload, t[1] FFT-CC, t[2] target preparation, t[3] IC-GN,
+ * t[0] target upload, t[1] FFT-CC, t[2] target preparation (the table, zeroed
+ * outputs; FFT-CC's per-reference pass on a reference's first frame), t[3] IC-GN,
  * t[4] result download, t[5] per-reference precompute (0 when cached). */
 TWDIC_API int twdic_frame_phase_times(const twdic_frame* h, float* t6);
 TWDIC_API int twdic_frame_destroy(twdic_frame* h);

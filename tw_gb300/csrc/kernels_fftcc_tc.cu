@@ -1738,8 +1738,8 @@ cudaError_t launch_one_size(TcJobsT<MULTI ? kMaxTcJobs : 1>& J, const FftccJob* 
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem_bytes);
     if (e != cudaSuccess) return e;
     // fewer batches than the SMs' groups: groups spread over half of the SMs
-    // (36 batches of 20x20 windows: 27 us in 36 CTAs of one group, 33 us in 8 of
-    // five).  Over all of them a launch of 277 batches is 4 us faster still, but
+    // (36 batches of 20x20 windows, before a batch held more than eight POIs:
+    // 27 us in 36 CTAs of one group, 33 us in 8 of five).  Over all of them a launch of 277 batches is 4 us faster still, but
     // keeps other streams' kernels off every SM.
     const int spread = (2 * nb + sms - 1) / sms;
     if (spread < s.groups) {
