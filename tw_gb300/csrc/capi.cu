@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -138,7 +139,13 @@ void grid_positions(const twdic_params& p, int nx, int ny, int32_t* yx) {
 }
 
 // -------------------------------------------------------------- Engine ----
+uint64_t next_serial() {
+    static std::atomic<uint64_t> last{0};
+    return ++last;
+}
+
 struct Engine {
+    const uint64_t serial = next_serial();  // no two handles of a process share one
     twdic_params prm{};
     Geom g{};
     int n = 0;  // POIs of the handle
@@ -1223,6 +1230,29 @@ FrameOut frame_out(Engine& e, const BatchArgs& a, int i) {
     return o;
 }
 
+// What a captured graph of this call depends on: the frames (by serial number,
+// a new handle may have the address of a destroyed one), their settings that
+// batch_enqueue reads, the caller's arrays, and what the launches' parameters
+// hold of the frames' state: the per-frame table, which other samplers
+// reallocate, the reference spectra and the shape of the tensor maps, which a
+// call of the frame alone may encode anew for its own tuning (the box widths
+// are launch parameters, the maps are read from memory at each replay).
+std::vector<uintptr_t> batch_key(const BatchArgs& a) {
+    std::vector<uintptr_t> key{(uintptr_t)a.count};
+    for (int i = 0; i < a.count; ++i) {
+        const Engine& e = a.frames[i]->e;
+        for (uintptr_t x : {(uintptr_t)a.frames[i], (uintptr_t)e.serial, (uintptr_t)e.guess, (uintptr_t)e.interp,
+                            (uintptr_t)e.fftcc_tune.use_tc, (uintptr_t)e.d_lut.p, (uintptr_t)e.c_fspec.p,
+                            (uintptr_t)e.tcmaps.key, (uintptr_t)a.tars[i],
+                            (uintptr_t)(a.strides ? a.strides[i] : 0), (uintptr_t)a.u[i], (uintptr_t)a.v[i],
+                            (uintptr_t)(a.zncc ? a.zncc[i] : nullptr), (uintptr_t)(a.p6 ? a.p6[i] : nullptr),
+                            (uintptr_t)(a.iters ? a.iters[i] : nullptr),
+                            (uintptr_t)(a.flags ? a.flags[i] : nullptr)})
+            key.push_back(x);
+    }
+    return key;
+}
+
 // The sampler a fast-path frame runs with under the batch's launch shape:
 // B-spline frames read the neighbourhood table with the B-spline weights, or
 // the B-spline LUT (the window sampler is Catmull-Rom only).
@@ -1514,22 +1544,14 @@ int twdic_batch_process(twdic_batch* b, int32_t count, twdic_frame* const* frame
     std::vector<uintptr_t> key;
     bool caches_ok = true;
     if (graphable) {
-        key.push_back((uintptr_t)count);
         for (int i = 0; i < count; ++i) {
             const Engine& e = frames[i]->e;
             caches_ok = caches_ok && e.cache_valid;
             // tensor-core FFT-CC frames read the reference spectra
             if (e.prm.path == TWDIC_PATH_FAST && e.fftcc_tune.use_tc && !e.guess && fftcc_tc_supported(e.g))
                 caches_ok = caches_ok && e.fspec_valid;
-            // the frame's own settings that batch_enqueue reads, then its arrays
-            for (uintptr_t x : {(uintptr_t)frames[i], (uintptr_t)e.guess, (uintptr_t)e.interp,
-                                (uintptr_t)e.fftcc_tune.use_tc, (uintptr_t)tars[i],
-                                (uintptr_t)(strides ? strides[i] : 0),
-                                (uintptr_t)u[i], (uintptr_t)v[i], (uintptr_t)(zncc ? zncc[i] : nullptr),
-                                (uintptr_t)(p6 ? p6[i] : nullptr), (uintptr_t)(iters ? iters[i] : nullptr),
-                                (uintptr_t)(flags ? flags[i] : nullptr)})
-                key.push_back(x);
         }
+        key = batch_key(a);
     }
     int rc = TWDIC_OK;
     if (graphable && caches_ok && b->exec && key == b->key) {
@@ -1550,7 +1572,9 @@ int twdic_batch_process(twdic_batch* b, int32_t count, twdic_frame* const* frame
                 const int rc2 = batch_enqueue(b, a);
                 e = cudaStreamEndCapture(b->stream, &graph);
                 if (rc2 == TWDIC_OK && e == cudaSuccess && graph) {
-                    if (cudaGraphInstantiate(&b->exec, graph, 0) == cudaSuccess) b->key = key;
+                    // (the key as the call left the frames: it may have moved a
+                    // buffer or encoded tensor maps)
+                    if (cudaGraphInstantiate(&b->exec, graph, 0) == cudaSuccess) b->key = batch_key(a);
                     else b->exec = nullptr;
                 }
                 if (graph) cudaGraphDestroy(graph);
