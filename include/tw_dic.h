@@ -256,6 +256,12 @@ TWDIC_API int twdic_frame_set_fftcc_tuning(twdic_frame* h, int use_tc, int group
  * 8.9e-4 without, in ZNCC units, against a candidate window of 0.01). */
 TWDIC_API int twdic_frame_set_fftcc_twiddles(twdic_frame* h, int hi_lo);
 
+/* A failure on the host, for tests: the handle sees what it would if the last
+ * per-reference pass of its FFT-CC had given up on a bounded wait (the spectra
+ * are computed again by the next call; the next call with host results returns
+ * TWDIC_ERR_TIMEOUT). */
+TWDIC_API int twdic_frame_fail_reference_pass(twdic_frame* h);
+
 typedef struct {
     int32_t icgn_threads, icgn_ctas_per_sm, icgn_sampler;
     int32_t fftcc_use_tc, fftcc_groups, fftcc_pois_per_group;

@@ -41,7 +41,7 @@ EXPORTED = (
     "twdic_frame_create", "twdic_frame_num_pois", "twdic_frame_poi_positions", "twdic_frame_set_reference",
     "twdic_frame_process", "twdic_frame_set_stream", "twdic_frame_phase_times", "twdic_frame_destroy",
     "twdic_frame_table",
-    "twdic_frame_set_tuning", "twdic_frame_set_icgn_layout", "twdic_frame_set_icgn_unroll", "twdic_frame_set_guess_mode", "twdic_frame_set_fftcc_twiddles", "twdic_icgn_compute_noalloc",
+    "twdic_frame_set_tuning", "twdic_frame_set_icgn_layout", "twdic_frame_set_icgn_unroll", "twdic_frame_fail_reference_pass", "twdic_frame_set_guess_mode", "twdic_frame_set_fftcc_twiddles", "twdic_icgn_compute_noalloc",
     "twdic_batch_create", "twdic_batch_set_stream", "twdic_batch_set_tuning", "twdic_batch_set_icgn_layout", "twdic_batch_set_icgn_unroll", "twdic_batch_set_graph",
     "twdic_batch_process", "twdic_batch_phase_times", "twdic_batch_destroy", "twdic_frame_device_bytes",
     "twdic_server_create", "twdic_server_add_stream", "twdic_server_remove_stream", "twdic_server_set_reference",
@@ -157,6 +157,7 @@ def load():
         "twdic_frame_set_tuning": ([_VP, _I, _I, _I, _I], _I),
         "twdic_frame_set_icgn_layout": ([_VP, _I], _I),
         "twdic_frame_set_icgn_unroll": ([_VP, _I], _I),
+        "twdic_frame_fail_reference_pass": ([_VP], _I),
         "twdic_frame_set_guess_mode": ([_VP, _I], _I),
         "twdic_frame_set_fftcc_twiddles": ([_VP, _I], _I),
         "twdic_icgn_compute_noalloc": ([P, _VP, _VP, _VP, ctypes.c_int32, _VP, _VP, _VP, _VP, _VP, _VP], _I),

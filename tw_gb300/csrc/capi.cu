@@ -144,7 +144,21 @@ uint64_t next_serial() {
     return ++last;
 }
 
+// Pinned host memory.
+struct PinnedBuf {
+    void* p = nullptr;
+    PinnedBuf() = default;
+    PinnedBuf(const PinnedBuf&) = delete;
+    PinnedBuf& operator=(const PinnedBuf&) = delete;
+    ~PinnedBuf() {
+        if (p) cudaFreeHost(p);
+    }
+};
+
 struct Engine {
+    // (first, so freed last: cudaFree of the device buffers has waited for the
+    // copies that are still to read or write it)
+    PinnedBuf pinned;
     const uint64_t serial = next_serial();  // no two handles of a process share one
     twdic_params prm{};
     Geom g{};
@@ -174,20 +188,25 @@ struct Engine {
     DevBuf d_tcmaps;
     void* h_tcmaps = nullptr;
     // pinned words beside them that calls read back (an asynchronous copy into
-    // pageable memory would be staged): [0] error flags, [1] POIs changed
+    // pageable memory would be staged): [0] error flags, [1] POIs changed,
+    // [2] error flags of the last per-reference pass of FFT-CC (kNotYet until
+    // they have arrived)
     volatile unsigned* h_words = nullptr;
+    static constexpr unsigned kNotYet = 0x80000000u;
     TcMapInfo tcmaps{0, 0, 0};
     // per-reference cache of the tensor-core FFT-CC: the reference windows'
     // spectra and integer sums at the POIs (dropped with the IC-GN cache)
     DevBuf c_fspec, c_fsum;
     bool fspec_valid = false;
+    // a timeout of the per-reference pass: its device word is still set; no
+    // call has returned it yet
+    bool ref_err_set = false, ref_timeout_owed = false;
     cudaEvent_t ev[7] = {};
     cudaEvent_t ev_sync = nullptr;  // orders this handle's stream with a batch stream
     float last_times[6] = {0, 0, 0, 0, 0, 0};
     bool times_pending = false;
 
     ~Engine() {
-        if (h_tcmaps) cudaFreeHost(h_tcmaps);
         for (auto& e : ev)
             if (e) cudaEventDestroy(e);
         if (ev_sync) cudaEventDestroy(ev_sync);
@@ -222,12 +241,14 @@ struct Engine {
         TW_TRY(d_p6.ensure(sizeof(float) * 6 * (size_t)n));
         TW_TRY(d_iters.ensure(sizeof(int) * (size_t)n));
         TW_TRY(d_flags.ensure((size_t)n));
-        TW_TRY(d_err.ensure(sizeof(unsigned)));
+        TW_TRY(d_err.ensure(2 * sizeof(unsigned)));  // per-frame launches, the per-reference pass
         TW_TRY(d_work.ensure(sizeof(int) * 4));
         TW_TRY(d_tcmaps.ensure(kTcMapsBytes));
-        TW_CUDA(cudaMallocHost(&h_tcmaps, kTcMapsBytes + 2 * sizeof(unsigned)));
+        TW_CUDA(cudaMallocHost(&pinned.p, kTcMapsBytes + 3 * sizeof(unsigned)));
+        h_tcmaps = pinned.p;
         h_words = reinterpret_cast<unsigned*>(static_cast<char*>(h_tcmaps) + kTcMapsBytes);
-        TW_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(unsigned), stream));
+        h_words[2] = 0;
+        TW_CUDA(cudaMemsetAsync(d_err.p, 0, 2 * sizeof(unsigned), stream));
         // DFT twiddles exp(-2 pi i k / N) of the two window sizes, rounded once
         // from double (the FP32 SIMT FFT-CC kernel reads them)
         std::vector<float> tw(4 * 64, 0.f);
@@ -269,12 +290,33 @@ struct Engine {
         return TWDIC_OK;
     }
 
+    // Whether the reference spectra are there: not computed, or their pass gave
+    // up on a bounded wait (its flags come back without a synchronisation, so a
+    // call looks at what has arrived; calls that return host results have waited
+    // for them).  Such spectra are incomplete and are computed again.
+    bool spectra_ok() {
+        const unsigned w = h_words[2];
+        if (fspec_valid && w != kNotYet && (w & kErrTimeout)) {
+            fspec_valid = false;
+            ref_err_set = ref_timeout_owed = true;
+        }
+        return fspec_valid;
+    }
+    // A timeout of the per-reference pass that no call has returned.
+    bool take_ref_timeout() {
+        spectra_ok();
+        const bool owed = ref_timeout_owed;
+        ref_timeout_owed = false;
+        return owed;
+    }
+
     int check_err() {
         TW_CUDA(cudaMemcpyAsync(const_cast<unsigned*>(h_words), d_err.p, sizeof(unsigned), cudaMemcpyDeviceToHost,
                                 stream));
         TW_CUDA(cudaStreamSynchronize(stream));
-        if (h_words[0] & kErrTimeout) {
-            cudaMemsetAsync(d_err.p, 0, sizeof(unsigned), stream);
+        const bool ref = take_ref_timeout(), frame = (h_words[0] & kErrTimeout) != 0;
+        if (frame) cudaMemsetAsync(d_err.p, 0, sizeof(unsigned), stream);
+        if (ref || frame) {
             return fail(TWDIC_ERR_TIMEOUT, "a bounded device-side wait gave up");
         }
         return TWDIC_OK;
@@ -297,15 +339,20 @@ struct Engine {
     // The reference spectra of the tensor-core FFT-CC: once per reference
     // (and POI set), by the per-reference pass, on this handle's stream.
     int ensure_fspec(const FftccTune& tune) {
-        if (fspec_valid) return TWDIC_OK;
+        if (spectra_ok()) return TWDIC_OK;
         if (!have_ref) return fail(TWDIC_ERR_STATE, "FFT-CC needs a reference image");
         TW_TRY(c_fspec.ensure(fftcc_tc_spectrum_bytes(g, n)));
         TW_TRY(c_fsum.ensure(sizeof(int2) * (size_t)n));
         TW_TRY(ensure_tc_maps(tune));
+        unsigned* err = d_err.as<unsigned>() + 1;
+        if (ref_err_set) TW_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned), stream));
+        ref_err_set = false;
         TW_CUDA(launch_fftcc_tc(g, d_ref.as<uint8_t>(), d_tar.as<uint8_t>(), d_tcmaps.p, tcmaps.key, tcmaps.uw,
                                 tcmaps.utoff, c_fspec.as<uint32_t>(), c_fsum.as<int2>(), d_poi.as<int2>(), n, nullptr,
-                                nullptr, nullptr, nullptr, d_err.as<unsigned>(), d_work.as<int>() + 1, tune, stream,
-                                true));
+                                nullptr, nullptr, nullptr, err, d_work.as<int>() + 1, tune, stream, true));
+        h_words[2] = kNotYet;
+        TW_CUDA(cudaMemcpyAsync(const_cast<unsigned*>(h_words + 2), err, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                                stream));
         fspec_valid = true;
         return TWDIC_OK;
     }
@@ -914,6 +961,15 @@ int twdic_frame_set_guess_mode(twdic_frame* h, int mode) {
     return TWDIC_OK;
 }
 
+int twdic_frame_fail_reference_pass(twdic_frame* h) {
+    if (!h) return fail(TWDIC_ERR_INVALID_ARG, "NULL handle");
+    Engine& e = h->e;
+    if (!e.fspec_valid) return fail(TWDIC_ERR_STATE, "no reference spectra yet (process a frame first)");
+    TW_CUDA(cudaStreamSynchronize(e.stream));  // the pass's own flags have arrived
+    e.h_words[2] = kErrTimeout;
+    return TWDIC_OK;
+}
+
 int twdic_frame_set_icgn_unroll(twdic_frame* h, int unroll) {
     if (!h) return fail(TWDIC_ERR_INVALID_ARG, "NULL handle");
     if (unroll != 2 && unroll != 4 && unroll != 8) return fail(TWDIC_ERR_INVALID_ARG, "unroll must be 2, 4 or 8");
@@ -1328,8 +1384,10 @@ int batch_enqueue(twdic_batch* b, const BatchArgs& a) {
         if (fast) fast_ic.push_back(i);
         prep.push_back(pj);
     }
-    // the per-reference pass of a frame's FFT-CC runs on its own counters
-    for (int i : fast_tc) TW_TRY(a.frames[i]->e.ensure_fspec(b->fftcc_tune));
+    // the per-reference pass of a frame's FFT-CC runs on its own counters (and
+    // never in a capture: the spectra's state is looked at once per call)
+    for (int i : fast_tc)
+        if (timed) TW_TRY(a.frames[i]->e.ensure_fspec(b->fftcc_tune));
     for (size_t k0 = 0; k0 < prep.size(); k0 += kMaxPrepJobs) {
         PrepJobs P;
         P.counters = b->d_work.as<int>();
@@ -1353,7 +1411,6 @@ int batch_enqueue(twdic_batch* b, const BatchArgs& a) {
         for (size_t m = 0; m < fast_tc.size(); ++m) {
             const int i = fast_tc[m];
             Engine& e = a.frames[i]->e;
-            TW_TRY(e.ensure_fspec(b->fftcc_tune));
             TW_TRY(e.ensure_tc_maps(b->fftcc_tune));
             const FrameOut o = frame_out(e, a, i);
             jobs.push_back(FftccJob{e.g, e.d_tcmaps.p, e.tcmaps.key, e.tcmaps.uw, e.tcmaps.utoff,
@@ -1545,11 +1602,11 @@ int twdic_batch_process(twdic_batch* b, int32_t count, twdic_frame* const* frame
     bool caches_ok = true;
     if (graphable) {
         for (int i = 0; i < count; ++i) {
-            const Engine& e = frames[i]->e;
+            Engine& e = frames[i]->e;
             caches_ok = caches_ok && e.cache_valid;
             // tensor-core FFT-CC frames read the reference spectra
             if (e.prm.path == TWDIC_PATH_FAST && e.fftcc_tune.use_tc && !e.guess && fftcc_tc_supported(e.g))
-                caches_ok = caches_ok && e.fspec_valid;
+                caches_ok = e.spectra_ok() && caches_ok;
         }
         key = batch_key(a);
     }
@@ -1603,8 +1660,10 @@ int twdic_batch_process(twdic_batch* b, int32_t count, twdic_frame* const* frame
         unsigned h = 0;
         TW_CUDA(cudaMemcpyAsync(&h, b->d_err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, b->stream));
         TW_CUDA(cudaStreamSynchronize(b->stream));
-        if (h & kErrTimeout) {
-            cudaMemsetAsync(b->d_err.p, 0, sizeof(unsigned), b->stream);
+        bool ref = false;  // (their flags were copied on this stream, or on one it waited for)
+        for (int i = 0; i < count; ++i) ref = frames[i]->e.take_ref_timeout() || ref;
+        if (h & kErrTimeout) cudaMemsetAsync(b->d_err.p, 0, sizeof(unsigned), b->stream);
+        if (ref || (h & kErrTimeout)) {
             return fail(TWDIC_ERR_TIMEOUT, "a bounded device-side wait gave up");
         }
     }
