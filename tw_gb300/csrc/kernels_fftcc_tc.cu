@@ -70,6 +70,7 @@ constexpr float kCandZncc = 0.01f;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kTmemCols = 128;  // TMEM columns a group may use (its stride is the shape's tcols)
 constexpr unsigned kWaitLimit = 1u << 24;
+constexpr int kMaxSmem = 227 * 1024;  // shared memory of a CTA
 
 // The tensor maps of one image pair: boxes [N rows][uw bytes] holding the
 // windows of a batch whose POIs lie on one POI row.
@@ -1429,9 +1430,9 @@ bool make_shape(const Geom& g, const FftccTune& tune, TcShape& s) {
     s.win_bytes = round_up(s.utoff + N * s.uw + 16, 128);
     s.off_win = region;
     s.group_bytes = round_up(region + 2 * s.win_bytes, 1024);  // two window slots
-    // 227 KB per CTA, less the groups' state
+    // what a CTA may have, less the groups' state
     s.cta_bytes = max_pb(s.HP) == 16 ? kCtaBytes<16> : kCtaBytes<8>;
-    const int limit = 227 * 1024 - s.cta_bytes;
+    const int limit = kMaxSmem - s.cta_bytes;
     // TMEM: each group's widest accumulator (stage 1: tiles x 2 HP, stages 2
     // and 3: 2 NP, stage 4: tiles x NP), 96 columns up to N = 48, so five
     // groups share the 512 columns there, four above
@@ -1440,7 +1441,7 @@ bool make_shape(const Geom& g, const FftccTune& tune, TcShape& s) {
     if (tune.groups > 0) s.groups = std::min(s.groups, tune.groups);  // tuned group count
     if (s.groups < 1) return false;
     s.smem_bytes = s.cta_bytes + o + s.groups * s.group_bytes;
-    return s.smem_bytes <= 227 * 1024;
+    return s.smem_bytes <= kMaxSmem;
 }
 
 // Twiddle matrices B1, C2, S2, B4 (hi and lo FP16) in the no-swizzle K-major
@@ -1626,6 +1627,17 @@ int shape_index(const TcShape& s) {
     return -1;
 }
 
+// The limit of a kernel's dynamic shared memory is state of the kernel, not of
+// a launch, and one kernel serves several window sizes, grid steps and tunings:
+// always the most a CTA may have (the launch's own size decides how many fit),
+// so that no thread's launch lowers it under another's.
+template <class Kernel>
+cudaError_t allow_all_smem(Kernel kern) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+}
+
 // Jobs of several window sizes in one k_fftcc_tc_seg launch.  counters:
 // kMaxTcSegs ints of scratch.
 cudaError_t launch_segments(const FftccJob* jobs, int njobs, const FftccTune& tune, unsigned* err, int* counters,
@@ -1683,9 +1695,7 @@ cudaError_t launch_segments(const FftccJob* jobs, int njobs, const FftccTune& tu
         acc += work[k];
     }
     auto kern = tune.twiddle_lo ? k_fftcc_tc_seg<true> : k_fftcc_tc_seg<false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaError_t e = allow_all_smem(kern);
     if (e != cudaSuccess) return e;
     if (!zeroed) {
         e = cudaMemsetAsync(counters, 0, sizeof(int) * kMaxTcSegs, st);
@@ -1735,7 +1745,7 @@ cudaError_t launch_one_size(TcJobsT<MULTI ? kMaxTcJobs : 1>& J, const FftccJob* 
         default: return cudaErrorNotSupported;
     }
 #undef TWDIC_TC_CASE
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem_bytes);
+    cudaError_t e = allow_all_smem(kern);
     if (e != cudaSuccess) return e;
     // fewer batches than the SMs' groups: groups spread over half of the SMs
     // (36 batches of 20x20 windows, before a batch held more than eight POIs:
@@ -1746,8 +1756,6 @@ cudaError_t launch_one_size(TcJobsT<MULTI ? kMaxTcJobs : 1>& J, const FftccJob* 
         s.smem_bytes -= (s.groups - spread) * s.group_bytes;
         s.groups = spread;
     }
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (e != cudaSuccess) return e;
     // with one group per CTA, two CTAs share an SM when they fit
     const int threads = kThreads * s.groups;
     int occ = 1;

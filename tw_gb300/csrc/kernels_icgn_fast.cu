@@ -1220,10 +1220,11 @@ static cudaError_t launch_icgn_fast_t(const IcgnJobsT<MULTI ? kMaxJobs : 1>& J, 
     }
     const size_t smem =
         sizeof(float) * ((size_t)((S_max + 3) & ~3) + (SAMPLER == kSampWindow ? (size_t)ws_max * ws_max : 0));
+    // (at most 37 KB, radius 31 with the window: below the 48 KB that need no
+    // attribute, which another thread's launch of smaller subsets would lower)
+    if (smem > 40 * 1024) return cudaErrorInvalidValue;
     auto kern = k_icgn_fast<THREADS, SAMPLER, MULTI>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0, occ = 0;
     cudaGetDevice(&dev);

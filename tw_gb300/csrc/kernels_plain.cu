@@ -415,7 +415,11 @@ cudaError_t launch_fftcc_plain(const Geom& g, const uint8_t* ref, const uint8_t*
     if (n <= 0) return cudaSuccess;
     const int Ny = 2 * g.ry, Hx = g.rx + 1;
     const size_t smem = sizeof(float2) * (128 + 4 * (size_t)Ny * Hx);
-    cudaError_t e = cudaFuncSetAttribute(k_fftcc_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // one value for every window (radii up to 31): another thread's launch of
+    // smaller windows never lowers the limit between this call and the launch
+    constexpr int kMaxSmem = sizeof(float2) * (128 + 4 * 62 * 32);
+    if (smem > kMaxSmem) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(k_fftcc_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e != cudaSuccess) return e;
     k_fftcc_plain<<<n, kFftThreads, smem, st>>>(g, ref, tar, poi, n, tw, u, v, zncc, status);
     return cudaGetLastError();
