@@ -218,7 +218,12 @@ TWDIC_API int twdic_icgn_set_interpolation(twdic_icgn* h, int mode);
 TWDIC_API int twdic_frame_set_interpolation(twdic_frame* h, int mode);
 
 /* Launch-shape tuning of a frame handle (no counterpart in the reference;
- * set by the autotuner).  icgn_threads: 32, 64, 128 or 256 threads per IC-GN CTA;
+ * set by the autotuner).  A handle starts with 1024 threads, chunk 32, the
+ * neighbourhood table and loops unrolled by 8, and launches of up to 16 POIs
+ * per SM take a shape of their own; from the first of set_tuning,
+ * set_icgn_layout and set_icgn_unroll on, the shape that is set runs whatever
+ * the number of POIs.  All shapes give the same results.
+ * icgn_threads: 32, 64, 128 or 256 threads per IC-GN CTA, or 512 or 1024 with a chunk;
  * icgn_ctas_per_sm: persistent CTAs per SM (0 = occupancy limit);
  * icgn_sampler: target interpolation of the fast IC-GN, 0 = staged window,
  * 1 = per-frame bicubic coefficient LUT, 2 = per-frame 4x4 neighbourhood
@@ -270,6 +275,8 @@ typedef struct {
     int32_t icgn_chunk;      /* IC-GN work layout (twdic_frame_set_icgn_layout) */
     int32_t icgn_unroll;     /* IC-GN sample-loop unrolling (twdic_frame_set_icgn_unroll) */
 } twdic_tuning;
+/* (of a handle that set no shape, and of an autotuner's choice of that rule:
+ * the shape it starts with) */
 TWDIC_API int twdic_frame_get_tuning(const twdic_frame* h, twdic_tuning* out);
 /* Autotuner (no reference counterpart): times the FFT-CC tile shapes and the
  * IC-GN launch shapes, samplers and sample-loop unrolling on this handle's reference and the given

@@ -222,6 +222,7 @@ struct Engine {
         icgn_tune.threads = 1024;
         icgn_tune.chunk = 32;
         icgn_tune.sampler = kSampNbhd;
+        icgn_tune.by_count = 1;  // until a caller sets a shape
         g = make_geom(p);
         n = num_pois;
         TW_CUDA(cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking));
@@ -942,6 +943,7 @@ int twdic_frame_set_tuning(twdic_frame* h, int icgn_threads, int icgn_ctas_per_s
     if (icgn_sampler < kSampWindow || icgn_sampler > kSampNbhd)
         return fail(TWDIC_ERR_INVALID_ARG, "sampler must be 0 (window), 1 (LUT) or 2 (neighbourhood table)");
     h->e.icgn_tune.sampler = icgn_sampler;
+    h->e.icgn_tune.by_count = 0;
     h->e.fftcc_tune.use_tc = fftcc_use_tc;
     return TWDIC_OK;
 }
@@ -951,6 +953,7 @@ int twdic_frame_set_icgn_layout(twdic_frame* h, int chunk) {
     if (!h) return fail(TWDIC_ERR_INVALID_ARG, "NULL handle");
     if (chunk < 0) return fail(TWDIC_ERR_INVALID_ARG, "chunk must be >= 0");
     h->e.icgn_tune.chunk = chunk;
+    h->e.icgn_tune.by_count = 0;
     return TWDIC_OK;
 }
 
@@ -974,6 +977,7 @@ int twdic_frame_set_icgn_unroll(twdic_frame* h, int unroll) {
     if (!h) return fail(TWDIC_ERR_INVALID_ARG, "NULL handle");
     if (unroll != 2 && unroll != 4 && unroll != 8) return fail(TWDIC_ERR_INVALID_ARG, "unroll must be 2, 4 or 8");
     h->e.icgn_tune.unroll = unroll;
+    h->e.icgn_tune.by_count = 0;
     return TWDIC_OK;
 }
 
@@ -1040,7 +1044,9 @@ bool cached_tuning_valid(const twdic_tuning& c) {
            c.fftcc_pois_per_group >= 0;
 }
 
-bool cache_lookup(const char* path, const std::string& key, twdic_tuning* t) {
+// by_count: the line's eleventh value; lines of ten are from before it, when
+// the number of POIs always decided.
+bool cache_lookup(const char* path, const std::string& key, twdic_tuning* t, int* by_count) {
     FILE* f = path ? std::fopen(path, "r") : nullptr;
     if (!f) return false;
     char line[512];
@@ -1050,11 +1056,13 @@ bool cache_lookup(const char* path, const std::string& key, twdic_tuning* t) {
         if (std::strncmp(line, key.c_str(), k) != 0 || line[k] != ' ') continue;
         twdic_tuning c;
         std::memset(&c, 0, sizeof(c));
-        if (std::sscanf(line + k, " %d %d %d %d %d %d %d %d %f %f", &c.icgn_threads, &c.icgn_ctas_per_sm,
+        int bc = 1;
+        if (std::sscanf(line + k, " %d %d %d %d %d %d %d %d %f %f %d", &c.icgn_threads, &c.icgn_ctas_per_sm,
                         &c.icgn_sampler, &c.icgn_chunk, &c.icgn_unroll, &c.fftcc_use_tc, &c.fftcc_groups,
-                        &c.fftcc_pois_per_group, &c.fftcc_ms, &c.icgn_ms) == 10 &&
-            cached_tuning_valid(c)) {
+                        &c.fftcc_pois_per_group, &c.fftcc_ms, &c.icgn_ms, &bc) >= 10 &&
+            cached_tuning_valid(c) && (bc == 0 || bc == 1)) {
             *t = c;  // the last entry for a key wins
+            *by_count = bc;
             found = true;
         }
     }
@@ -1080,12 +1088,14 @@ int twdic_frame_autotune(twdic_frame* h, const uint8_t* tar, int32_t stride, int
     const std::string key = tuning_key(e);
     twdic_tuning t;
     std::memset(&t, 0, sizeof(t));
-    if (cache_lookup(cache_path, key, &t)) {
+    int by_count = 0;
+    if (cache_lookup(cache_path, key, &t, &by_count)) {
         e.icgn_tune.threads = t.icgn_threads;
         e.icgn_tune.ctas_per_sm = t.icgn_ctas_per_sm;
         e.icgn_tune.sampler = t.icgn_sampler;
         e.icgn_tune.chunk = t.icgn_chunk;
         e.icgn_tune.unroll = t.icgn_unroll;
+        e.icgn_tune.by_count = by_count;
         e.fftcc_tune.use_tc = t.fftcc_use_tc;
         e.fftcc_tune.groups = t.fftcc_groups;
         e.fftcc_tune.pois_per_group = t.fftcc_pois_per_group;
@@ -1144,17 +1154,26 @@ int twdic_frame_autotune(twdic_frame* h, const uint8_t* tar, int32_t stride, int
     IcgnTune best_i = icgn0;
     float best_ims = 1e30f, fms = best_fms;
     if (e.prm.path == TWDIC_PATH_FAST) {
-        // (threads, chunk): one POI per warp over runs of consecutive POIs,
-        // then one POI per CTA
-        const int shapes[][2] = {{1024, 32}, {1024, 64}, {512, 32}, {32, 0}, {64, 0}, {128, 0}, {256, 0}};
+        // (threads, chunk, by the number of POIs): the shape of handles that set
+        // none, where that is another one; one POI per warp over runs of
+        // consecutive POIs (runs of up to 64 only where 32 are exceeded); then
+        // one POI per CTA
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const int shapes[][3] = {{1024, 32, 1}, {1024, 32, 0}, {1024, 64, 0}, {512, 32, 0},
+                                 {32, 0, 0},    {64, 0, 0},    {128, 0, 0},   {256, 0, 0}};
         for (const auto& sh : shapes) {
             for (int sampler : {kSampNbhd, kSampLut, kSampWindow}) {
                 if (sh[1] > 0 && sampler == kSampWindow) continue;
+                if (sh[1] == 64 && e.n <= 32 * (long long)sms) continue;
                 IcgnTune c;
                 c.threads = sh[0];
                 c.chunk = sh[1];
                 c.ctas_per_sm = 0;
                 c.sampler = sampler;
+                c.by_count = sh[2];
+                if (c.by_count && !icgn_shape_by_count(c, e.n)) continue;
                 e.icgn_tune = c;
                 float f = 0, ic = 0;
                 const int rc = measure(&f, &ic);
@@ -1171,7 +1190,7 @@ int twdic_frame_autotune(twdic_frame* h, const uint8_t* tar, int32_t stride, int
             }
         }
         // sample-loop unrolling of the chosen one-POI-per-warp shape
-        if (best_i.chunk > 0 && best_i.threads == 1024) {
+        if (best_i.chunk > 0 && best_i.threads == 1024 && !best_i.by_count) {
             for (int unroll : {2, 4}) {
                 IcgnTune c = best_i;
                 c.unroll = unroll;
@@ -1210,9 +1229,9 @@ int twdic_frame_autotune(twdic_frame* h, const uint8_t* tar, int32_t stride, int
     if (cache_path) {
         FILE* f = std::fopen(cache_path, "a");
         if (f) {
-            std::fprintf(f, "%s %d %d %d %d %d %d %d %d %.4f %.4f\n", key.c_str(), t.icgn_threads,
+            std::fprintf(f, "%s %d %d %d %d %d %d %d %d %.4f %.4f %d\n", key.c_str(), t.icgn_threads,
                          t.icgn_ctas_per_sm, t.icgn_sampler, t.icgn_chunk, t.icgn_unroll, t.fftcc_use_tc,
-                         t.fftcc_groups, t.fftcc_pois_per_group, t.fftcc_ms, t.icgn_ms);
+                         t.fftcc_groups, t.fftcc_pois_per_group, t.fftcc_ms, t.icgn_ms, best_i.by_count);
             std::fclose(f);
         }
     }
@@ -1515,6 +1534,7 @@ int twdic_batch_create(twdic_batch** out) {
     b->tune.threads = 1024;
     b->tune.chunk = 32;
     b->tune.sampler = kSampNbhd;
+    b->tune.by_count = 1;  // until a caller sets a shape
     *out = b.release();
     return TWDIC_OK;
 }
@@ -1535,6 +1555,7 @@ int twdic_batch_set_tuning(twdic_batch* b, int icgn_threads, int icgn_ctas_per_s
     b->tune.threads = icgn_threads;
     b->tune.ctas_per_sm = icgn_ctas_per_sm;
     b->tune.sampler = icgn_sampler;
+    b->tune.by_count = 0;
     if (b->exec) cudaGraphExecDestroy(b->exec);
     b->exec = nullptr;
     b->key.clear();
@@ -1545,6 +1566,7 @@ int twdic_batch_set_icgn_layout(twdic_batch* b, int chunk) {
     if (!b) return fail(TWDIC_ERR_INVALID_ARG, "NULL handle");
     if (chunk < 0) return fail(TWDIC_ERR_INVALID_ARG, "chunk must be >= 0");
     b->tune.chunk = chunk;
+    b->tune.by_count = 0;
     if (b->exec) cudaGraphExecDestroy(b->exec);
     b->exec = nullptr;
     b->key.clear();
@@ -1555,6 +1577,7 @@ int twdic_batch_set_icgn_unroll(twdic_batch* b, int unroll) {
     if (!b) return fail(TWDIC_ERR_INVALID_ARG, "NULL handle");
     if (unroll != 2 && unroll != 4 && unroll != 8) return fail(TWDIC_ERR_INVALID_ARG, "unroll must be 2, 4 or 8");
     b->tune.unroll = unroll;
+    b->tune.by_count = 0;
     if (b->exec) cudaGraphExecDestroy(b->exec);
     b->exec = nullptr;
     b->key.clear();

@@ -27,7 +27,12 @@ struct IcgnTune {
     // 1024, a table sampler); 0: one POI per CTA
     int chunk = 0;
     int unroll = 8;  // sample-loop unrolling of the one-POI-per-warp kernel (2, 4 or 8)
+    // 1: nobody asked for a shape, launches of a few POIs per SM may take
+    // another one (launch_icgn_jobs); 0: the shape above is the one that runs
+    int by_count = 0;
 };
+// whether by_count replaces a shape for a launch of n POIs
+bool icgn_shape_by_count(const IcgnTune& tune, long long n);
 
 // Image pairs (jobs) of one batched IC-GN launch: each job has its own
 // geometry, images, POI set, reference cache and outputs.  The table is a

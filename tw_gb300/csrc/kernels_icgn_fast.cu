@@ -1336,6 +1336,33 @@ static bool icgn_warp_eligible(const Jobs& J, const IcgnTune& tune) {
     return true;
 }
 
+// The 32-warp CTAs (one per SM, 64 registers) are for launches that fill them.
+// Fewer POIs leave a warp's own latency in the open: up to 16 per SM, CTAs of
+// four warps at 128 registers, whose sample steps overlap more, and up to four
+// per SM the team kernel.  IC-GN of one frame (us, POIs every 8 px, 152 SMs:
+// the lines lie at 608 and 2,432 POIs), team / four-warp / 32-warp:
+//            17x17 subsets     27x27             41x41              61x61
+//   289 POIs  43 /  45 /  51    29 /  37 /  39    29 /  37 /  43     51 /  76 / 100
+//   600       46 /  47 /  51    27 /  31 /  33    35 /  51 /  47     66 / 104 / 104
+//   900       57 /  51 /  70    37 /  37 /  41    57 /  45 /  51    111 /  88 /  98
+//   2,401     96 /  64 /  72    70 /  45 /  54   113 /  55 /  70    221 / 107 / 135
+//   3,600    123 /  78 /  84   100 /  59 /  59   162 /  90 /  82    320 / 182 / 164
+// The same order holds for calls of three streams in turn, where 600 POIs of
+// 17x17 to 61x61 subsets are a tie of the first two (36 / 36 to 69 / 71 us).
+constexpr int kTeamPois = 4, kFourWarpPois = 16;  // POIs per SM
+
+static int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+bool icgn_shape_by_count(const IcgnTune& tune, long long n) {
+    return tune.by_count && tune.chunk > 0 && tune.threads == 1024 &&
+           (tune.sampler == kSampNbhd || tune.sampler == kSampNbhdBs) && n <= (long long)kFourWarpPois * sm_count();
+}
+
 template <bool MULTI>
 static cudaError_t launch_icgn_jobs(const IcgnJobsT<MULTI ? kMaxJobs : 1>& J, int* work, const IcgnTune& tune,
                                     cudaStream_t st) {
@@ -1348,24 +1375,16 @@ static cudaError_t launch_icgn_jobs(const IcgnJobsT<MULTI ? kMaxJobs : 1>& J, in
     if (tune.sampler == kSampLut) { TWDIC_ICGN_WARP(NW, kSampLut); }                              \
     if (tune.sampler == kSampNbhdBs) { TWDIC_ICGN_WARP(NW, kSampNbhdBs); }                        \
     TWDIC_ICGN_WARP(NW, kSampNbhd)
-        // The 32-warp CTAs (one per SM, 64 registers) are for launches that
-        // fill them.  Fewer POIs leave a warp's own latency in the open: up to 16
-        // per SM, CTAs of four warps at 128 registers, whose sample steps overlap
-        // more (1,936 POIs, 33x33 subsets: 44 us against 50 us), and up to four
-        // per SM the team kernel (285 POIs, 21x21 subsets: 23 us against 33 us;
-        // 1,936 POIs: 75 us).
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const bool full = tune.threads == 1024 && tune.sampler != kSampLut;
-        if (full && J.total <= 4 * sms) {
+        // a shape that the caller set runs; otherwise few POIs take another one
+        const bool few = icgn_shape_by_count(tune, J.total);
+        if (few && J.total <= kTeamPois * sm_count()) {
 #define TWDIC_ICGN_TEAM(SA)                                                                                \
     return launch_icgn_team_t<8, SA, MULTI>(J, st)
             if (tune.sampler == kSampNbhdBs) { TWDIC_ICGN_TEAM(kSampNbhdBs); }
             TWDIC_ICGN_TEAM(kSampNbhd);
 #undef TWDIC_ICGN_TEAM
         }
-        if (tune.threads == 128 || (full && J.total <= 16 * sms)) { TWDIC_ICGN_WARP_N(4); }
+        if (tune.threads == 128 || few) { TWDIC_ICGN_WARP_N(4); }
         if (tune.threads == 256) { TWDIC_ICGN_WARP_N(8); }
         if (tune.threads == 512) { TWDIC_ICGN_WARP_N(16); }
         TWDIC_ICGN_WARP_N(32);
