@@ -1,5 +1,6 @@
 """A launch shape that the caller sets is the one that runs; the shapes chosen
 by the number of POIs are those of handles that set none."""
+import numpy as np
 import pytest
 
 from launches import launches
@@ -85,3 +86,19 @@ def test_autotuned_shape_by_the_number_of_pois(tmp_path):
         assert k.name == name, (values, k)
         if name == "k_icgn_warp":
             assert k.args[0] == "32" and k.args[3] == "2", k
+
+
+@pytest.mark.parametrize("r,step,twiddles", [(13, 25, 0), (13, 26, 0), (12, 29, 1), (15, 22, 1), (12, 3, 0)])
+def test_fftcc_groups_of_small_windows(r, step, twiddles):
+    """Five groups per CTA where five fit with eight POIs per batch, whatever
+    the POI step (a batch of more never costs a group)."""
+    nx = 64
+    side = 2 + 2 * r + 16 + step * (nx - 1)
+    f = dic.DICFrame(dic.make_params(side, side, 1, 1, side - 2, side - 2, r, r, step, step, 8, 8, 20, 0.001))
+    f.set_fftcc_twiddles(twiddles)
+    img = np.random.default_rng(r).integers(0, 255, (side, side), np.uint8)
+    f.set_reference(img)
+    o = f.alloc_outputs()
+    f.process(img, **o)
+    found = [x for x in launches(lambda: f.process(img, **o)) if x.name == "k_fftcc_tc"]
+    assert len(found) == 1 and found[0].threads == 640, found

@@ -56,8 +56,9 @@ namespace {
 constexpr int kThreads = 128;
 constexpr int kCandChunk = 128;   // exact re-evaluations per pass (all POIs of a group batch)
 // POIs per batch (upper bound) by HP: the small windows fill the 128 rows of
-// stages 2 and 3 with more than eight POIs (14 of 16x16, 9 of 24x24)
-constexpr int max_pb(int hp) { return hp <= 16 ? 16 : 8; }
+// stages 2 and 3 with more than eight POIs (16 of up to 14x14, 14 of 16x16,
+// 9 of 24x24)
+constexpr int max_pb(int hp) { return hp <= 8 ? 16 : (hp <= 16 ? 14 : 8); }
 constexpr int kMaxGroups = 5;     // 128-thread groups per CTA (upper bound; window sizes up to 48)
 constexpr int kSegGroups = 4;     // groups per CTA of the larger windows and of the segmented kernel
 // Candidate window of the approximate correlation surface, in ZNCC units.
@@ -349,7 +350,7 @@ struct TcCta : TcHead {
     int wsm[kMaxGroups][2];
 };
 template <int PBM>
-constexpr int kCtaBytes = ((int)sizeof(TcCta<PBM>) + 1023) / 1024 * 1024;
+constexpr int kCtaBytes = ((int)sizeof(TcCta<PBM>) + 127) / 128 * 128;
 
 // The tensor maps of jobs [lo, hi): visible to the tensor-map proxy (they
 // were written to device memory by copies) and prefetched.  Thread 0 of each
@@ -1346,7 +1347,9 @@ __global__ void __launch_bounds__(128 * kSegGroups, 1) k_fftcc_tc_seg(const __gr
 // ----------------------------------------------------------- host side ----
 int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
-bool make_shape(const Geom& g, const FftccTune& tune, TcShape& s) {
+// The shape with at most `most` POIs per batch; fit: the groups that the SM has
+// room for.
+bool make_shape_of(const Geom& g, const FftccTune& tune, int most, TcShape& s, int& fit) {
     if (g.rx != g.ry) return false;
     const int N = 2 * g.rx;
     if (N < 8 || N > 64) return false;
@@ -1357,7 +1360,7 @@ bool make_shape(const Geom& g, const FftccTune& tune, TcShape& s) {
     // POIs per batch: the (POI, ky) rows of stages 2 and 3 fill one 128-row
     // tile; the (POI, x) rows of stages 1 and 4 take up to two, each with its
     // own TMEM columns (2 HP at stage 1, NP at stage 4) within the group's 128
-    int pb = std::min(128 / s.H, max_pb(s.HP));
+    int pb = std::min(std::min(128 / s.H, max_pb(s.HP)), most);
     // beyond eight only as long as one box holds the batch's windows
     if (g.grid_x > 0) pb = std::min(pb, std::max(8, (256 - 15 - N) / g.grid_x + 1));
     if (tune.pois_per_group > 0) pb = std::min(pb, tune.pois_per_group);  // tuned batch size
@@ -1429,19 +1432,31 @@ bool make_shape(const Geom& g, const FftccTune& tune, TcShape& s) {
     s.utoff = round_up(N * s.uw, 128);
     s.win_bytes = round_up(s.utoff + N * s.uw + 16, 128);
     s.off_win = region;
-    s.group_bytes = round_up(region + 2 * s.win_bytes, 1024);  // two window slots
+    s.group_bytes = round_up(region + 2 * s.win_bytes, 128);  // two window slots
     // what a CTA may have, less the groups' state
-    s.cta_bytes = max_pb(s.HP) == 16 ? kCtaBytes<16> : kCtaBytes<8>;
+    s.cta_bytes = max_pb(s.HP) == 16 ? kCtaBytes<16> : (max_pb(s.HP) == 14 ? kCtaBytes<14> : kCtaBytes<8>);
     const int limit = kMaxSmem - s.cta_bytes;
     // TMEM: each group's widest accumulator (stage 1: tiles x 2 HP, stages 2
     // and 3: 2 NP, stage 4: tiles x NP), 96 columns up to N = 48, so five
     // groups share the 512 columns there, four above
     s.tcols = round_up(std::max(std::max(s.tiles1 * 2 * s.HP, s.tiles4 * s.NP), 2 * s.NP), 32);
-    s.groups = std::min(std::min(kMaxGroups, 512 / s.tcols), (limit - o) / s.group_bytes);
+    s.groups = fit = std::min(std::min(kMaxGroups, 512 / s.tcols), (limit - o) / s.group_bytes);
     if (tune.groups > 0) s.groups = std::min(s.groups, tune.groups);  // tuned group count
     if (s.groups < 1) return false;
     s.smem_bytes = s.cta_bytes + o + s.groups * s.group_bytes;
     return s.smem_bytes <= kMaxSmem;
+}
+
+// A batch of more than eight POIs (small windows) has wider boxes: not where
+// that costs a group (26x26 windows every 25 px: five groups of 8 or four of 9).
+// By the groups that fit, whatever number is tuned: the maps of a frame serve
+// launches of its own and of batches, which run four groups.
+bool make_shape(const Geom& g, const FftccTune& tune, TcShape& s) {
+    int fit = 0, fit8 = 0;
+    if (!make_shape_of(g, tune, max_pb(0), s, fit)) return false;
+    TcShape s8;
+    if (s.PB > 8 && tune.pois_per_group == 0 && make_shape_of(g, tune, 8, s8, fit8) && fit8 > fit) s = s8;
+    return true;
 }
 
 // Twiddle matrices B1, C2, S2, B4 (hi and lo FP16) in the no-swizzle K-major
