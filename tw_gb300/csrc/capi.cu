@@ -188,19 +188,17 @@ struct Engine {
     DevBuf d_tcmaps;
     void* h_tcmaps = nullptr;
     // pinned words beside them that calls read back (an asynchronous copy into
-    // pageable memory would be staged): [0] error flags, [1] POIs changed,
-    // [2] error flags of the last per-reference pass of FFT-CC (kNotYet until
-    // they have arrived)
+    // pageable memory would be staged): [0] error flags, [1] POIs changed; and
+    // [2] error flags of FFT-CC's per-reference pass, which the kernel writes
+    // here itself, only when it gives up (ref_err: the device's address)
     volatile unsigned* h_words = nullptr;
-    static constexpr unsigned kNotYet = 0x80000000u;
+    unsigned* ref_err = nullptr;
     TcMapInfo tcmaps{0, 0, 0};
     // per-reference cache of the tensor-core FFT-CC: the reference windows'
     // spectra and integer sums at the POIs (dropped with the IC-GN cache)
     DevBuf c_fspec, c_fsum;
     bool fspec_valid = false;
-    // a timeout of the per-reference pass: its device word is still set; no
-    // call has returned it yet
-    bool ref_err_set = false, ref_timeout_owed = false;
+    bool ref_timeout_owed = false;  // a timeout of the per-reference pass that no call has returned
     cudaEvent_t ev[7] = {};
     cudaEvent_t ev_sync = nullptr;  // orders this handle's stream with a batch stream
     float last_times[6] = {0, 0, 0, 0, 0, 0};
@@ -242,14 +240,15 @@ struct Engine {
         TW_TRY(d_p6.ensure(sizeof(float) * 6 * (size_t)n));
         TW_TRY(d_iters.ensure(sizeof(int) * (size_t)n));
         TW_TRY(d_flags.ensure((size_t)n));
-        TW_TRY(d_err.ensure(2 * sizeof(unsigned)));  // per-frame launches, the per-reference pass
+        TW_TRY(d_err.ensure(sizeof(unsigned)));
         TW_TRY(d_work.ensure(sizeof(int) * 4));
         TW_TRY(d_tcmaps.ensure(kTcMapsBytes));
         TW_CUDA(cudaMallocHost(&pinned.p, kTcMapsBytes + 3 * sizeof(unsigned)));
         h_tcmaps = pinned.p;
         h_words = reinterpret_cast<unsigned*>(static_cast<char*>(h_tcmaps) + kTcMapsBytes);
         h_words[2] = 0;
-        TW_CUDA(cudaMemsetAsync(d_err.p, 0, 2 * sizeof(unsigned), stream));
+        TW_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&ref_err), const_cast<unsigned*>(h_words + 2), 0));
+        TW_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(unsigned), stream));
         // DFT twiddles exp(-2 pi i k / N) of the two window sizes, rounded once
         // from double (the FP32 SIMT FFT-CC kernel reads them)
         std::vector<float> tw(4 * 64, 0.f);
@@ -291,15 +290,15 @@ struct Engine {
         return TWDIC_OK;
     }
 
-    // Whether the reference spectra are there: not computed, or their pass gave
-    // up on a bounded wait (its flags come back without a synchronisation, so a
-    // call looks at what has arrived; calls that return host results have waited
-    // for them).  Such spectra are incomplete and are computed again.
+    // Whether the reference spectra are there, as far as the host knows: spectra
+    // of a pass that gave up on a bounded wait are incomplete and are computed
+    // again (a call looks without a synchronisation; those that return host
+    // results have waited for the pass).
     bool spectra_ok() {
-        const unsigned w = h_words[2];
-        if (fspec_valid && w != kNotYet && (w & kErrTimeout)) {
+        if (h_words[2] & kErrTimeout) {
+            h_words[2] = 0;
             fspec_valid = false;
-            ref_err_set = ref_timeout_owed = true;
+            ref_timeout_owed = true;
         }
         return fspec_valid;
     }
@@ -345,15 +344,9 @@ struct Engine {
         TW_TRY(c_fspec.ensure(fftcc_tc_spectrum_bytes(g, n)));
         TW_TRY(c_fsum.ensure(sizeof(int2) * (size_t)n));
         TW_TRY(ensure_tc_maps(tune));
-        unsigned* err = d_err.as<unsigned>() + 1;
-        if (ref_err_set) TW_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned), stream));
-        ref_err_set = false;
         TW_CUDA(launch_fftcc_tc(g, d_ref.as<uint8_t>(), d_tar.as<uint8_t>(), d_tcmaps.p, tcmaps.key, tcmaps.uw,
                                 tcmaps.utoff, c_fspec.as<uint32_t>(), c_fsum.as<int2>(), d_poi.as<int2>(), n, nullptr,
-                                nullptr, nullptr, nullptr, err, d_work.as<int>() + 1, tune, stream, true));
-        h_words[2] = kNotYet;
-        TW_CUDA(cudaMemcpyAsync(const_cast<unsigned*>(h_words + 2), err, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                                stream));
+                                nullptr, nullptr, nullptr, ref_err, d_work.as<int>() + 1, tune, stream, true));
         fspec_valid = true;
         return TWDIC_OK;
     }
@@ -968,7 +961,7 @@ int twdic_frame_fail_reference_pass(twdic_frame* h) {
     if (!h) return fail(TWDIC_ERR_INVALID_ARG, "NULL handle");
     Engine& e = h->e;
     if (!e.fspec_valid) return fail(TWDIC_ERR_STATE, "no reference spectra yet (process a frame first)");
-    TW_CUDA(cudaStreamSynchronize(e.stream));  // the pass's own flags have arrived
+    TW_CUDA(cudaStreamSynchronize(e.stream));  // the pass has ended
     e.h_words[2] = kErrTimeout;
     return TWDIC_OK;
 }
@@ -1683,7 +1676,7 @@ int twdic_batch_process(twdic_batch* b, int32_t count, twdic_frame* const* frame
         unsigned h = 0;
         TW_CUDA(cudaMemcpyAsync(&h, b->d_err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, b->stream));
         TW_CUDA(cudaStreamSynchronize(b->stream));
-        bool ref = false;  // (their flags were copied on this stream, or on one it waited for)
+        bool ref = false;  // (their passes ran on this stream, or on one it waited for)
         for (int i = 0; i < count; ++i) ref = frames[i]->e.take_ref_timeout() || ref;
         if (h & kErrTimeout) cudaMemsetAsync(b->d_err.p, 0, sizeof(unsigned), b->stream);
         if (ref || (h & kErrTimeout)) {
