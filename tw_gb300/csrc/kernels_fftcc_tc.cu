@@ -23,11 +23,14 @@
 // correlation), with the reference's first-maximum rule.
 // ZNCC is the quotient of the exact integer sums, evaluated in FP32.
 //
-// Up to five groups of 128 threads (one warpgroup each, each with the TMEM
-// columns of its widest accumulator: 96 up to N = 48, then 128, so five groups
-// there and four above) per CTA, one CTA per SM, persistent over batches of
-// POIs; thread 0
-// of a group issues its MMAs, completion is signalled through an mbarrier
+// Up to five groups of 128 threads (one warpgroup each) per CTA, one CTA per
+// SM, persistent over batches of POIs.  How many: up to N = 30 the five of the
+// launch bounds (a group takes 64 TMEM columns or fewer and 22 to 32 KB up to
+// steps of 11 px: TMEM and shared memory would hold more); from N = 32 to 46,
+// at 96 columns a group, the five that TMEM holds, or the four that shared
+// memory holds at wider POI steps (N = 40: from 6 px); above, at 128 columns,
+// at most four, and by shared memory mostly three (N = 48 from 5 px) or two (N =
+// 60 from 8 px).  Thread 0 of a group issues its MMAs, completion is signalled through an mbarrier
 // (bounded wait), the epilogues read TMEM with tcgen05.ld.  The reference
 // windows' spectra are computed once per reference (the per-reference pass)
 // and read back by the per-frame pass, which transforms the target windows
@@ -59,7 +62,7 @@ constexpr int kCandChunk = 128;   // exact re-evaluations per pass (all POIs of 
 // stages 2 and 3 with more than eight POIs (16 of up to 14x14, 14 of 16x16,
 // 9 of 24x24)
 constexpr int max_pb(int hp) { return hp <= 8 ? 16 : (hp <= 16 ? 14 : 8); }
-constexpr int kMaxGroups = 5;     // 128-thread groups per CTA (upper bound; window sizes up to 48)
+constexpr int kMaxGroups = 5;     // 128-thread groups per CTA (upper bound: 96 registers a thread)
 constexpr int kSegGroups = 4;     // groups per CTA of the larger windows and of the segmented kernel
 // Candidate window of the approximate correlation surface, in ZNCC units.
 // The exact peak lies within twice the surface's error of the approximate
@@ -83,7 +86,7 @@ constexpr int kMaxTcSegs = kMaxTcSegsScratch;    // window sizes per launch (N =
 
 struct TcShape {
     int N, H, HP, NP, PB, tiles1, K4, groups;
-    int tcols;      // TMEM columns per group (96 or 128): the widest accumulator of the four stages
+    int tcols;      // TMEM columns per group (32 to 128): the widest accumulator of the four stages
     int uw, utoff;  // one-row boxes: width (0: none for this geometry) and the target box's offset
     int win_bytes;  // a group's window region
     int cta_bytes;  // the CTA's shared state, before the tables
@@ -1437,8 +1440,8 @@ bool make_shape_of(const Geom& g, const FftccTune& tune, int most, TcShape& s, i
     s.cta_bytes = max_pb(s.HP) == 16 ? kCtaBytes<16> : (max_pb(s.HP) == 14 ? kCtaBytes<14> : kCtaBytes<8>);
     const int limit = kMaxSmem - s.cta_bytes;
     // TMEM: each group's widest accumulator (stage 1: tiles x 2 HP, stages 2
-    // and 3: 2 NP, stage 4: tiles x NP), 96 columns up to N = 48, so five
-    // groups share the 512 columns there, four above
+    // and 3: 2 NP, stage 4: tiles x NP): 32 columns up to N = 14, 64 up to 30,
+    // 96 up to 46 (five groups share the 512), then 128
     s.tcols = round_up(std::max(std::max(s.tiles1 * 2 * s.HP, s.tiles4 * s.NP), 2 * s.NP), 32);
     s.groups = fit = std::min(std::min(kMaxGroups, 512 / s.tcols), (limit - o) / s.group_bytes);
     if (tune.groups > 0) s.groups = std::min(s.groups, tune.groups);  // tuned group count
@@ -1763,9 +1766,10 @@ cudaError_t launch_one_size(TcJobsT<MULTI ? kMaxTcJobs : 1>& J, const FftccJob* 
     cudaError_t e = allow_all_smem(kern);
     if (e != cudaSuccess) return e;
     // fewer batches than the SMs' groups: groups spread over half of the SMs
-    // (36 batches of 20x20 windows, before a batch held more than eight POIs:
-    // 27 us in 36 CTAs of one group, 33 us in 8 of five).  Over all of them a launch of 277 batches is 4 us faster still, but
-    // keeps other streams' kernels off every SM.
+    // (26 batches of 20x20 windows: 18 us in 26 CTAs of one group, 24 us in six
+    // of five; 277 of 32x32: 28 us in 70 of four, 30 us in 56).  Over all of
+    // them the 277 take 26 us, but three streams in turn gain nothing (43.5 and
+    // 43.7 us a frame) and a launch would keep others off every SM.
     const int spread = (2 * nb + sms - 1) / sms;
     if (spread < s.groups) {
         s.smem_bytes -= (s.groups - spread) * s.group_bytes;

@@ -1242,7 +1242,8 @@ static cudaError_t launch_icgn_fast_t(const IcgnJobsT<MULTI ? kMaxJobs : 1>& J, 
 }
 
 int icgn_fast_residency(const Geom& g, const IcgnTune& tune) {
-    // one POI per warp: no per-POI shared memory, one residency for all
+    // one POI per warp: no per-POI shared memory, so one value for all frames
+    // (a batch sorts its frames by it; the launchers ask for the real occupancy)
     if (tune.chunk > 0 && tune.sampler != kSampWindow && tune.threads >= 128) return 32 * 32 / tune.threads;
     const int S = (2 * g.rx + 1) * (2 * g.ry + 1), ws = icgn_fast_window(g);
     const size_t smem = sizeof(float) * ((size_t)((S + 3) & ~3) + (tune.sampler == kSampWindow ? (size_t)ws * ws : 0));
@@ -1275,17 +1276,21 @@ cudaError_t launch_ref_grad(const Geom& g, const uint8_t* ref, float2* grad, cud
 }
 
 // unroll: the sample loops' blocks, 2, 4 or 8 steps for the one-CTA-per-SM shape
-// (2048^2, 41x41 subsets: 2.23 ms by 8, 2.24 by 6, 2.23 by 10, 2.27 by 16), 4 for
-// CTAs of fewer warps.
+// (2048^2, 41x41 subsets: 2.23 ms by 8, 2.30 by 4, 2.41 by 2, 2.24 by 6, 2.23 by
+// 10, 2.27 by 16), 4 for CTAs of fewer warps.  Those are for few POIs; asked for
+// on that frame, beside 2.29 ms (155,236 POIs): 16 warps 2.51, 8 warps 2.64, four
+// (128 registers a thread, four CTAs per SM) 2.77 ms.
 template <int NW, int SAMPLER, bool MULTI>
 static cudaError_t launch_icgn_warp_t(const IcgnJobsT<MULTI ? kMaxJobs : 1>& J, int chunk, int ctas_per_sm, int unroll,
                                       cudaStream_t st) {
     auto kern = k_icgn_warp<NW, SAMPLER, MULTI, 4>;
     if (NW == 32 && unroll == 2) kern = k_icgn_warp<NW, SAMPLER, MULTI, (NW == 32 ? 2 : 4)>;
     if (NW == 32 && unroll == 8) kern = k_icgn_warp<NW, SAMPLER, MULTI, (NW == 32 ? 8 : 4)>;
-    // shared memory for the resident CTAs (up to 8 KB each with the runtime's
-    // 1 KB; at a share of 0 the smaller CTAs are not all resident), the rest of
-    // the SM's 256 KB to L1
+    // shared memory for the resident CTAs (400 B a warp and the runtime's 1 KB:
+    // 13.8, 7.4, 4.2 and 2.6 KB for CTAs of 32, 16, 8 and four warps), the rest
+    // of the SM's 256 KB to L1.  A share of 0 is the smallest that holds one
+    // CTA, so not all of the smaller ones would be resident (four warps on the
+    // frame above, at 0: 4.6 ms)
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, NW == 32 ? 0 : 10);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0, occ = 0;

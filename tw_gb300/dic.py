@@ -275,7 +275,8 @@ class DICFrame:
 
     def set_tuning(self, icgn_threads=128, icgn_ctas_per_sm=0, icgn_sampler=0, fftcc_use_tc=1, icgn_chunk=0):
         """icgn_sampler: SAMPLER_WINDOW, SAMPLER_LUT or SAMPLER_NBHD;
-        icgn_chunk: the IC-GN work layout (set_icgn_layout; None keeps it)."""
+        icgn_chunk: the IC-GN work layout (set_icgn_layout; None keeps it).
+        The shape that is set runs whatever the number of POIs."""
         check(self._lib.twdic_frame_set_tuning(self._h, icgn_threads, icgn_ctas_per_sm, icgn_sampler,
                                                fftcc_use_tc))
         if icgn_chunk is not None:
