@@ -342,7 +342,9 @@ TWDIC_API int twdic_icgn_compute_noalloc(const twdic_params* p, const uint8_t* d
  * frames and arrays equal the previous call's replays a CUDA graph captured
  * from that call (one cudaGraphLaunch; `*replayed` = 1).  Inputs are read
  * from the same device arrays, so the caller refreshes their contents
- * between calls. */
+ * between calls.  A frame's new reference or setting, or a call of it alone
+ * that moved its table or tensor maps, makes the next call run and be
+ * captured anew. */
 typedef struct twdic_batch twdic_batch;
 TWDIC_API int twdic_batch_create(twdic_batch** out);
 TWDIC_API int twdic_batch_set_stream(twdic_batch* b, void* stream);

@@ -5,22 +5,16 @@ import re
 import tempfile
 from collections import namedtuple
 
+import pytest
+
 Launch = namedtuple("Launch", "name args threads blocks registers shared")
 _started = False
 
 
-def launches(call):
-    """Runs `call` and returns its launches of this library's kernels in order:
-    kernel name, template arguments as texts, threads per block, blocks,
-    registers per thread and shared memory per block."""
+def _kernels(call):
+    """The kernel events of a profiled session around `call`."""
     import torch
     from torch.profiler import ProfilerActivity, profile
-    global _started
-    if not _started:  # a process's first session may miss launches
-        with profile(activities=[ProfilerActivity.CUDA]):
-            torch.zeros(1, device="cuda").add_(1)
-            torch.cuda.synchronize()
-        _started = True
     torch.cuda.synchronize()
     with profile(activities=[ProfilerActivity.CUDA]) as prof:
         call()
@@ -33,12 +27,28 @@ def launches(call):
             events = json.load(f)["traceEvents"]
     finally:
         os.unlink(path)
+    return sorted((e for e in events if e.get("cat") == "kernel"), key=lambda e: e["ts"])
+
+
+def launches(call):
+    """Runs `call` and returns its launches of this library's kernels in order:
+    kernel name, template arguments as texts, threads per block, blocks,
+    registers per thread and shared memory per block.  Skips the test where the
+    profiling interface reports nothing (another tool may hold it)."""
+    import torch
+    global _started
+    if not _started:  # (a process's first session may miss launches)
+        probe = torch.zeros(1, device="cuda")
+        _kernels(lambda: probe.add_(1))
+        if not _kernels(lambda: probe.add_(1)):
+            pytest.skip("no kernel records from the CUDA profiling interface")
+        _started = True
     out = []
-    for e in sorted((e for e in events if e.get("cat") == "kernel"), key=lambda e: e["ts"]):
+    for e in _kernels(call):
         m = re.search(r"\b(k_\w+)(?:<([^()]*(?:\(\w+\)[^()]*)*)>)?\(", e["name"])
         if not m:
             continue
-        args = [re.sub(r"^\(\w+\)", "", a.strip()) for a in (m.group(2) or "").split(",")] if m.group(2) else []
+        args = [re.sub(r"^\(\w+\)", "", x.strip()) for x in m.group(2).split(",")] if m.group(2) else []
         a = e["args"]
         prod = lambda d: d[0] * d[1] * d[2]  # noqa: E731
         out.append(Launch(m.group(1), args, prod(a["block"]), prod(a["grid"]), a["registers per thread"],
